@@ -537,7 +537,7 @@ INST_PER_UNIT = {"p2g_cells_kernel": 575950823 / 5767168,
 
 # The smoother's sweep kernels (one of them runs, by element type, halo and
 # active-set size).
-SWEEP_KERNELS = ("sweep_compact_kernel", "sweep_pipe_kernel", "sweep_phase_kernel", "sweep_wave_kernel")
+SWEEP_KERNELS = ("sweep_compact_kernel", "sweep_phase_kernel", "sweep_wave_kernel")
 
 
 def sweep_kernel_time(kern):

@@ -16,7 +16,7 @@ struct SweepPlan {
     size_t n = 0;
     int color_off[9] = {0};
     DevBuf nbr;    // int32 [n][27]
-    DevBuf bxyz;   // int32 [n][3]
+    DevBuf bxyz;   // int32 [n][8]: block coordinates, flags, mirrored sides
     DevBuf order;  // int32 [n] plan indices grouped by colour
     // Slots whose x-faces the sweep reads (x-neighbours of active blocks, as
     // faces or edges), for the x-face side buffer (see sweep.cu).
