@@ -241,16 +241,19 @@ __global__ void p2g_gather_kernel(const float* pos, const float* vel, const floa
     }
 }
 
-// Particles a splat warp stages at once (two float4 each): a whole typical
-// tile where the FP64 window leaves room in shared memory, 32 otherwise.
-template <int BSX, int M> struct SplatCap {
-    static constexpr int v = 2 * 8 * (BSX + 2 * M) * (BSX + 2 * M) * (BSX + 2 * M) <= 131072 ? 128 : 32;
+// Launch shape of the general splat kernel.  Tiles wait for their overlapping
+// predecessors, so more warps in a CTA mostly wait longer.  16^3 blocks have
+// 512 tiles: 20 warps, one CTA per SM (fastest among 16, 20, 24 and 32 on
+// B200), staging a whole typical tile per warp where the FP64 window leaves
+// room.  8^3 blocks have 64 tiles, of which two or three can run at a time, so
+// small CTAs share an SM instead (with one CTA of 20 warps per SM, B200, 4.8 M
+// particles in 8^3 blocks: r_p = 1 1.92 against 0.58 ms, 2.5 46.9 against 10.1 ms,
+// 3 46.9 against 18.2 ms).
+template <int BSX, int M> struct SplatShape {
+    static constexpr int WARPS = BSX == 8 ? 8 : 20;
+    static constexpr int CTAS = BSX == 8 ? 3 : 1;  // per SM
+    static constexpr int CAP = BSX == 8 ? 64 : 2 * 8 * (BSX + 2 * M) * (BSX + 2 * M) * (BSX + 2 * M) <= 131072 ? 128 : 32;
 };
-
-// Warps of a splat CTA.  Tiles wait for their overlapping predecessors, so
-// more warps mostly wait longer; 20 (one CTA per SM, up to 96 registers a
-// thread) measured fastest on B200 among 16, 20, 24 and 32.
-constexpr int kSplatWarps = 20;
 
 // Pairs of f32 in one 64-bit register, and the paired IEEE single-precision
 // operations of sm_100 (each half rounded to nearest, exactly as the scalar
@@ -281,7 +284,7 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
     return r;
 }
 
-// Splat kernel: one CTA per (particle block, direction DIR).  The block's
+// Splat kernel: one CTA per (particle block, direction).  The block's
 // (bsx + 2M)^3 staging window of face sums lives in shared memory in FP64.
 // Cells are grouped in 2x2x2 tiles; a warp takes a whole tile (its 8 cells in
 // a fixed order).  The face windows of two tiles overlap only when the tiles
@@ -293,70 +296,76 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
 // contributions in colour order, then cell order: a fixed summation order
 // with no atomics and no CTA-wide barrier between colours.
 //
-// Inside a cell, the lanes of the warp take the (2M+1)^2 positions of the
-// cell's face window across the two axes other than the face axis, and each
-// lane keeps the 2M+1 faces along the face axis in FP64 registers.  For every
-// particle of the cell (sorted order) a lane evaluates the reference's f32
-// term for each of its faces inside the particle's clipped footprint
-// (p2g.rs:263-330, operation by operation; the footprint arrives as the
-// particle's lane and face bits), then adds its register sums to the window.
+// Inside a tile, a group of RW^2 lanes takes a cell: the RW x RW rows of the
+// cell's face window across the two axes other than the face axis, RW being
+// the rows that a footprint of this radius covers unless a coordinate lies
+// exactly on a cell centre (compact_rows), so with RW = 3 a warp works on
+// three cells at once (4.2 M particles in 16^3 blocks, r_p = 1.5, B200: 1.86 ms
+// with 25 rows of which 9 carry weight, 0.91 ms with 3 x 9; 5.6 M in 8^3
+// blocks 8.64 -> 1.71 ms with the smaller CTAs).  Each lane keeps the 2M+1 faces along
+// the face axis in FP64 registers.  For every particle of its cell (sorted
+// order) it evaluates the reference's f32 term for each of its faces inside
+// the particle's clipped footprint (p2g.rs:263-330, operation by operation;
+// the footprint arrives as the particle's lane and face bits), then the groups
+// add their register sums to the window in cell order.  Rows of a footprint
+// beyond the RW x RW ones (a particle exactly on a cell centre) are added by
+// the whole warp after the cells.
 // A tile wait that runs past a second sets bit 4 of the status word and goes
 // on (the result is then wrong and the host reports the error).
-template <int BSX, int M, int DIR>
-__global__ void __launch_bounds__(32 * kSplatWarps, 1) p2g_cells_kernel(SplatArgs a) {
+template <int M, int RW> struct CellLanes {
+    static constexpr int WIN = 2 * M + 1;
+    static constexpr int CO = (WIN - RW) / 2;   // first of the RW rows in the window of WIN
+    static constexpr int NRW = RW * RW;
+    static constexpr int Q = (NRW + 31) / 32;   // lane rounds of one cell
+    static constexpr int G = NRW > 32 ? 1 : 32 / NRW;  // cells at once
+    // lane bits of the window outside the RW x RW rows
+    static constexpr uint64_t outside() {
+        uint64_t m = 0;
+        for (int v = 0; v < WIN; ++v)
+            for (int u = 0; u < WIN; ++u)
+                if (u < CO || u >= CO + RW || v < CO || v >= CO + RW) m |= 1ull << (u + WIN * v);
+        return m;
+    }
+};
+
+template <int BSX, int M, int RW, int DIR>
+__device__ __forceinline__ void splat_cells_body(const SplatArgs& a, const int k_pb, double* st, uint32_t* s_done,
+                                                 const uint16_t* s_order, uint32_t* s_next, int n_tiles) {
+    using L = CellLanes<M, RW>;
     constexpr int W = BSX + 2 * M;
     constexpr int WW = W * W * W;
-    constexpr int WIN = 2 * M + 1;
-    constexpr int NUV = WIN * WIN;       // lane positions
-    constexpr int Q = (NUV + 31) / 32;   // lane rounds
-    constexpr int T = BSX / 2, K = M + 1, NT = T * T * T;
+    constexpr int WIN = L::WIN;
+    constexpr int T = BSX / 2, K = M + 1;
     constexpr int NNB = WIN * WIN * WIN;  // tile offsets in [-M, M]^3
-    constexpr int CAP = SplatCap<BSX, M>::v;
+    constexpr int CAP = SplatShape<BSX, M>::CAP;
     constexpr int NR = (NNB + 31) / 32;   // of them per lane
     // Faces s = 1 .. WIN-1 in pairs; face 0 (offset -M-1) is inside a
     // particle's footprint only when the particle sits exactly on a face
     // plane, so it is evaluated alone, and only for such particles.
     constexpr int NP = (WIN - 1) / 2;    // face pairs (2h+1, 2h+2)
-    static_assert(WIN <= 7 && NUV <= 56, "lane and face bits must fit one u64");
-    static_assert(NT < 0xffff, "tile indices must fit 16 bits");
-    extern __shared__ double st[];       // [2][W^3]: mass, momentum; then per-warp particle slots
-    __shared__ uint32_t s_done[NT];
-    __shared__ uint16_t s_order[NT];     // tiles in colour-major order
-    __shared__ uint32_t s_next;
-    const int k_pb = blockIdx.x;
+    static_assert(WIN <= 7, "lane and face bits must fit one u64");
     const int tid = threadIdx.x, lane = tid & 31;
-    float4* wslot = reinterpret_cast<float4*>(st + 2 * WW) + (size_t)(tid >> 5) * 2 * SplatCap<BSX, M>::v;
-    for (int i = tid; i < 2 * WW; i += blockDim.x) st[i] = 0.0;
-    for (int t = tid; t < NT; t += blockDim.x) {
-        s_done[t] = 0;
-        const int tx = t % T, ty = (t / T) % T, tz = t / (T * T);
-        const int cx = tx % K, cy = ty % K, cz = tz % K;
-        const int ci = cx + K * (cy + K * cz);
-        int base = 0;
-        for (int c = 0; c < ci; ++c) {
-            const int ox = c % K, oy = (c / K) % K, oz = c / (K * K);
-            base += ((T - ox + K - 1) / K) * ((T - oy + K - 1) / K) * ((T - oz + K - 1) / K);
-        }
-        const int ntx = (T - cx + K - 1) / K, nty = (T - cy + K - 1) / K;
-        s_order[base + (tx / K) + ntx * ((ty / K) + nty * (tz / K))] = (uint16_t)t;
-    }
-    if (tid == 0) s_next = 0;
+    float4* wslot = reinterpret_cast<float4*>(st + 2 * WW) + (size_t)(tid >> 5) * 2 * CAP;
     const uint64_t key = a.pb_key[k_pb];
     const int32_t b0[3] = {(int32_t)compact3(key) * BSX, (int32_t)compact3(key >> 1) * BSX,
                            (int32_t)compact3(key >> 2) * BSX};
     // axes: F = face axis (registers), U and V = lane axes
     constexpr int F = DIR, U = DIR == 0 ? 1 : 0, V = DIR == 2 ? 1 : 2;
+    constexpr int kStride[3] = {1, W, W * W};  // window index step per axis
     const int32_t* cb = a.cell_begin + (size_t)k_pb * BSX * BSX * BSX;
     const int32_t* ce = a.cell_end + (size_t)k_pb * BSX * BSX * BSX;
     const float* __restrict__ pv = a.pv[DIR];
     const uint64_t* __restrict__ lmask = a.lane_mask[DIR];
     const float inv_r2 = a.inv_r2;
-    __syncthreads();
+    // this lane's cell of a round (>= G: idle).  With one cell at a time every
+    // lane belongs to it, those beyond its rows included, so that the loop
+    // bounds below are the same for the whole warp.
+    const int grp = L::G == 1 ? 0 : lane / L::NRW;
     while (true) {
         uint32_t q = 0;
-        if (lane == 0) q = atomicAdd(&s_next, 1u);
+        if (lane == 0) q = atomicAdd(s_next, 1u);
         q = __shfl_sync(0xffffffffu, q, 0);
-        if (q >= (uint32_t)NT) break;
+        if (q >= (uint32_t)n_tiles) break;
         const int t = s_order[q];
         const int tc[3] = {t % T, (t / T) % T, t / (T * T)};
         const int ci = tc[0] % K + K * (tc[1] % K + K * (tc[2] % K));
@@ -369,7 +378,7 @@ __global__ void __launch_bounds__(32 * kSplatWarps, 1) p2g_cells_kernel(SplatArg
         }
         // the overlapping tiles of lower colours: each lane takes up to NR of
         // them; the warp waits for them before its first shared-memory add
-        // of this tile (so the tile's first cell is computed meanwhile),
+        // of this tile (so the tile's first cells are computed meanwhile),
         // drops each as it is seen done, and sleeps between rounds
         uint32_t nbi[(NR + 1) / 2];  // tile indices, two 16-bit fields per word, 0xffff = none
 #pragma unroll
@@ -411,141 +420,183 @@ __global__ void __launch_bounds__(32 * kSplatWarps, 1) p2g_cells_kernel(SplatArg
             __threadfence_block();
             deps_pending = false;
         };
-        const int e_tile = (int)__reduce_max_sync(0xffffffffu, lane < 8 ? (uint32_t)cend : 0u);
-        int st_lo = 0, st_hi = 0;  // the particles held by the warp's staging slots
-        for (int sub = 0; sub < 8; ++sub) {
-            // cells of a tile have overlapping face windows: order this
-            // cell's shared-memory updates after the previous cell's across
-            // the warp's lanes
-            __syncwarp();
-            const int b = __shfl_sync(0xffffffffu, cbeg, sub), e = __shfl_sync(0xffffffffu, cend, sub);
-            if (b >= e) continue;
-            int cell[3];
-            cell[0] = 2 * tc[0] + (sub & 1);
-            cell[1] = 2 * tc[1] + ((sub >> 1) & 1);
-            cell[2] = 2 * tc[2] + (sub >> 2);
+        // the tile's particles are one contiguous range of the sorted order
+        // (its 8 cells are Morton neighbours; empty cells have an empty range)
+        const bool has = lane < 8 && cbeg < cend;
+        const int t_beg = (int)__reduce_min_sync(0xffffffffu, has ? (uint32_t)cbeg : 0x7fffffffu);
+        const int t_end = (int)__reduce_max_sync(0xffffffffu, has ? (uint32_t)cend : 0u);
+        for (int s0 = t_beg; s0 < t_end; s0 += CAP) {
+            // stage up to CAP of them with coalesced loads; the cells read
+            // their particles by broadcast
+            const int s1 = min(s0 + CAP, t_end);
+            __syncwarp();  // the previous chunk's readers are done
+            bool odd = false;
 #pragma unroll
-            for (int qq = 0; qq < Q; ++qq) {
-                const int uv = lane + 32 * qq;
-                const bool on = uv < NUV;
-                // staging coordinates of this lane's row: U, V offsets in [-M, M]
-                const int su = cell[U] + (uv % WIN), sv = cell[V] + (uv / WIN);
-                const float gu = (float)(b0[U] - M + su), gv = (float)(b0[V] - M + sv);
-                // face positions along F, in pairs: staging cell[F] + s - 1
-                uint64_t gf2[NP];
-#pragma unroll
-                for (int h = 0; h < NP; ++h)
-                    gf2[h] = f2_pack((float)(b0[F] - M + cell[F] + 2 * h), (float)(b0[F] - M + cell[F] + 2 * h + 1));
-                const float gf0 = (float)(b0[F] - M + cell[F] - 1);
-                double am[WIN], av[WIN];
-#pragma unroll
-                for (int s = 0; s < WIN; ++s) am[s] = av[s] = 0.0;
-                // the cell's particles from the warp's staging slots, which
-                // hold up to CAP consecutive particles of the tile (the 8 cells
-                // of a tile are one contiguous range of the sorted order):
-                // staged with coalesced loads, CAP / 32 per lane, then read by
-                // broadcast
-                for (int p0 = b; p0 < e;) {
-                  if (p0 < st_lo || p0 >= st_hi) {
-                      __syncwarp();
-                      st_lo = p0;
-                      st_hi = min(p0 + CAP, e_tile);
-#pragma unroll
-                      for (int k = 0; k < CAP / 32; ++k) {
-                          const int pl = st_lo + lane + 32 * k;
-                          if (pl < st_hi) {
-                              const uint64_t f = lmask[pl];
-                              const float m = a.pm[pl];
-                              const size_t q = (size_t)pl * a.ps;
-                              const float pc[3] = {a.px[q] - 0.5f, a.py[q] - 0.5f, a.pz[q] - 0.5f};
-                              wslot[pl - st_lo] = make_float4(pc[U], pc[V], pc[F], m);
-                              wslot[CAP + pl - st_lo] = make_float4(m * pv[q], __uint_as_float((uint32_t)f),
-                                                                    __uint_as_float((uint32_t)(f >> 32)), 0.0f);
-                          }
-                      }
-                      __syncwarp();
-                  }
-                  const int pend = min(e, st_hi);
-                  for (int j = p0; j < pend; ++j) {
-                    const float4 P = wslot[j - st_lo];        // U, V, F coordinates (minus 0.5), mass
-                    const float4 R = wslot[CAP + j - st_lo];  // momentum, lane bits (low, high)
-                    const uint32_t f_lo = __float_as_uint(R.y), f_hi = __float_as_uint(R.z);
-                    // bit s: face s inside the footprint, none when the lane's
-                    // row is outside it (no branch: the warp stays converged,
-                    // and a zero weight adds +0 to a sum that starts at +0)
-                    const uint32_t lanebit = on ? (((qq == 0 ? f_lo : f_hi) >> lane) & 1u) : 0u;
-                    const uint32_t fbits = (f_hi >> 24) & (0u - lanebit);
-                    const float m_p = P.w, scale_mom = R.x;
-                    const float du = gu - P.x, dv = gv - P.y;
-                    const uint64_t pf2 = f2_pack(P.z, P.z);
-                    // p2g.rs:287-325: dz2 = dz*dz; dyz = dz2 + dy*dy; dist_sq = dx*dx + dyz,
-                    // with (dx, dy, dz) = (df, du, dv), (du, df, dv) or (du, dv, df)
-                    float hoist0 = 0.0f, hoist1 = 0.0f;
-                    if (DIR == 0) hoist0 = dv * dv + du * du;  // dyz
-                    else if (DIR == 1) { hoist0 = dv * dv; hoist1 = du * du; }  // dz2, dx*dx
-                    else { hoist0 = dv * dv; hoist1 = du * du; }                // dy*dy, dx*dx
-                    const uint64_t h02 = f2_pack(hoist0, hoist0), h12 = f2_pack(hoist1, hoist1);
-#pragma unroll
-                    for (int h = 0; h < NP; ++h) {
-                        const uint64_t df = f2_sub(gf2[h], pf2);
-                        // products that feed a sum stay scalar: a paired
-                        // product feeding a paired sum may be contracted
-                        float d0, d1;
-                        f2_unpack(df, d0, d1);
-                        const uint64_t sq = f2_pack(d0 * d0, d1 * d1);
-                        uint64_t dist;
-                        if (DIR == 0) dist = f2_add(sq, h02);                 // dx*dx + dyz
-                        else if (DIR == 1) dist = f2_add(h12, f2_add(h02, sq));  // dx*dx + (dz2 + dy*dy)
-                        else dist = f2_add(h12, f2_add(sq, h02));             // dx*dx + (dz2 + dy*dy)
-                        const uint64_t df2 = f2_add(f2_add(dist, df), f2_pack(0.25f, 0.25f));
-                        float e0, e1;
-                        f2_unpack(df2, e0, e1);
-                        const uint64_t t = f2_sub(f2_pack(1.0f, 1.0f), f2_pack(e0 * inv_r2, e1 * inv_r2));
-                        float w0, w1;
-                        f2_unpack(t, w0, w1);
-                        w0 = ((fbits >> (2 * h + 1)) & 1u) ? fmaxf(w0, 0.0f) : 0.0f;
-                        w1 = ((fbits >> (2 * h + 2)) & 1u) ? fmaxf(w1, 0.0f) : 0.0f;
-                        uint64_t w = f2_pack(w0, w1);
-                        w = f2_mul(f2_mul(w, w), w);
-                        float tm0, tm1, tv0, tv1;
-                        f2_unpack(f2_mul(w, f2_pack(m_p, m_p)), tm0, tm1);
-                        f2_unpack(f2_mul(w, f2_pack(scale_mom, scale_mom)), tv0, tv1);
-                        am[2 * h + 1] += (double)tm0;
-                        av[2 * h + 1] += (double)tv0;
-                        am[2 * h + 2] += (double)tm1;
-                        av[2 * h + 2] += (double)tv1;
-                    }
-                    if ((f_hi >> 24) & 1u) {  // face 0: the same for every lane of the warp
-                        const float df = gf0 - P.z;
-                        const float sq = df * df;
-                        float dist;
-                        if (DIR == 0) dist = sq + hoist0;
-                        else if (DIR == 1) dist = hoist1 + (hoist0 + sq);
-                        else dist = hoist1 + (sq + hoist0);
-                        const float df2 = (dist + df) + 0.25f;
-                        float w = 1.0f - df2 * inv_r2;
-                        w = (fbits & 1u) ? fmaxf(w, 0.0f) : 0.0f;
-                        w = (w * w) * w;
-                        am[0] += (double)(w * m_p);
-                        av[0] += (double)(w * scale_mom);
-                    }
-                  }
-                  p0 = pend;
+            for (int k = 0; k < CAP / 32; ++k) {
+                const int pl = s0 + lane + 32 * k;
+                if (pl < s1) {
+                    const uint64_t f = lmask[pl];
+                    const float m = a.pm[pl];
+                    const size_t qq = (size_t)pl * a.ps;
+                    const float pc[3] = {a.px[qq] - 0.5f, a.py[qq] - 0.5f, a.pz[qq] - 0.5f};
+                    wslot[pl - s0] = make_float4(pc[U], pc[V], pc[F], m);
+                    wslot[CAP + pl - s0] = make_float4(m * pv[qq], __uint_as_float((uint32_t)f),
+                                                       __uint_as_float((uint32_t)(f >> 32)), 0.0f);
+                    odd = odd || (f & L::outside()) != 0;
                 }
-                if (deps_pending) wait_deps();
-                if (on) {
+            }
+            odd = __any_sync(0xffffffffu, odd);
+            __syncwarp();
+#pragma unroll 1
+            for (int c0 = 0; c0 < 8; c0 += L::G) {
+                // this lane's cell of the round and its particles of the chunk
+                const int sub = c0 + grp;
+                const int bq = max(__shfl_sync(0xffffffffu, cbeg, sub & 7), s0);
+                const int eq = min(__shfl_sync(0xffffffffu, cend, sub & 7), s1);
+                const int cnt = grp < L::G && sub < 8 ? max(eq - bq, 0) : 0;
+                const int rounds = L::G == 1 ? cnt : (int)__reduce_max_sync(0xffffffffu, (uint32_t)cnt);
+                if (!rounds) continue;
+                const int cell[3] = {2 * tc[0] + (sub & 1), 2 * tc[1] + ((sub >> 1) & 1), 2 * tc[2] + ((sub >> 2) & 1)};
 #pragma unroll
-                    for (int s = 0; s < WIN; ++s) {
-                        const int sf = cell[F] + s - 1;
-                        if (sf < 0 || sf >= W) continue;
-                        int sc[3];
-                        sc[F] = sf;
-                        sc[U] = su;
-                        sc[V] = sv;
-                        const int si = (sc[2] * W + sc[1]) * W + sc[0];
-                        st[si] += am[s];
-                        st[WW + si] += av[s];
+                for (int qr = 0; qr < L::Q; ++qr) {
+                    const int row = L::G == 1 ? lane + 32 * qr : lane - grp * L::NRW;
+                    const bool on = cnt > 0 && row < L::NRW;
+                    // this lane's row: offsets in the window of WIN along U and V
+                    const int du0 = L::CO + row % RW, dv0 = L::CO + row / RW, bit = du0 + WIN * dv0;
+                    const int su = cell[U] + du0, sv = cell[V] + dv0;
+                    const float gu = (float)(b0[U] - M + su), gv = (float)(b0[V] - M + sv);
+                    // face positions along F, in pairs: staging cell[F] + s - 1
+                    uint64_t gf2[NP];
+#pragma unroll
+                    for (int h = 0; h < NP; ++h)
+                        gf2[h] = f2_pack((float)(b0[F] - M + cell[F] + 2 * h), (float)(b0[F] - M + cell[F] + 2 * h + 1));
+                    const float gf0 = (float)(b0[F] - M + cell[F] - 1);
+                    double am[WIN], av[WIN];
+#pragma unroll
+                    for (int s = 0; s < WIN; ++s) am[s] = av[s] = 0.0;
+#pragma unroll 1
+                    for (int j = 0; j < rounds; ++j) {
+                        const bool live = on && j < cnt;
+                        // (a lane whose cell has fewer particles repeats its last with weight zero)
+                        const int at = on ? bq - s0 + min(j, cnt - 1) : 0;
+                        const float4 P = wslot[at];        // U, V, F coordinates (minus 0.5), mass
+                        const float4 R = wslot[CAP + at];  // momentum, lane bits (low, high)
+                        const uint32_t f_lo = __float_as_uint(R.y), f_hi = __float_as_uint(R.z);
+                        // bit s: face s inside the footprint, none when the lane's
+                        // row is outside it (no branch: the warp stays converged,
+                        // and a zero weight adds +0 to a sum that starts at +0)
+                        const uint32_t lanebit = live ? (((WIN * WIN <= 32 || bit < 32 ? f_lo : f_hi) >> (bit & 31)) & 1u) : 0u;
+                        const uint32_t fbits = (f_hi >> 24) & (0u - lanebit);
+                        const float m_p = P.w, scale_mom = R.x;
+                        const float du = gu - P.x, dv = gv - P.y;
+                        const uint64_t pf2 = f2_pack(P.z, P.z);
+                        // p2g.rs:287-325: dz2 = dz*dz; dyz = dz2 + dy*dy; dist_sq = dx*dx + dyz,
+                        // with (dx, dy, dz) = (df, du, dv), (du, df, dv) or (du, dv, df)
+                        float hoist0 = 0.0f, hoist1 = 0.0f;
+                        if (DIR == 0) hoist0 = dv * dv + du * du;  // dyz
+                        else if (DIR == 1) { hoist0 = dv * dv; hoist1 = du * du; }  // dz2, dx*dx
+                        else { hoist0 = dv * dv; hoist1 = du * du; }                // dy*dy, dx*dx
+                        const uint64_t h02 = f2_pack(hoist0, hoist0), h12 = f2_pack(hoist1, hoist1);
+#pragma unroll
+                        for (int h = 0; h < NP; ++h) {
+                            const uint64_t df = f2_sub(gf2[h], pf2);
+                            // products that feed a sum stay scalar: a paired
+                            // product feeding a paired sum may be contracted
+                            float d0, d1;
+                            f2_unpack(df, d0, d1);
+                            const uint64_t sq = f2_pack(d0 * d0, d1 * d1);
+                            uint64_t dist;
+                            if (DIR == 0) dist = f2_add(sq, h02);                 // dx*dx + dyz
+                            else if (DIR == 1) dist = f2_add(h12, f2_add(h02, sq));  // dx*dx + (dz2 + dy*dy)
+                            else dist = f2_add(h12, f2_add(sq, h02));             // dx*dx + (dz2 + dy*dy)
+                            const uint64_t df2 = f2_add(f2_add(dist, df), f2_pack(0.25f, 0.25f));
+                            float e0, e1;
+                            f2_unpack(df2, e0, e1);
+                            const uint64_t tt = f2_sub(f2_pack(1.0f, 1.0f), f2_pack(e0 * inv_r2, e1 * inv_r2));
+                            float w0, w1;
+                            f2_unpack(tt, w0, w1);
+                            w0 = ((fbits >> (2 * h + 1)) & 1u) ? fmaxf(w0, 0.0f) : 0.0f;
+                            w1 = ((fbits >> (2 * h + 2)) & 1u) ? fmaxf(w1, 0.0f) : 0.0f;
+                            uint64_t w = f2_pack(w0, w1);
+                            w = f2_mul(f2_mul(w, w), w);
+                            float tm0, tm1, tv0, tv1;
+                            f2_unpack(f2_mul(w, f2_pack(m_p, m_p)), tm0, tm1);
+                            f2_unpack(f2_mul(w, f2_pack(scale_mom, scale_mom)), tv0, tv1);
+                            am[2 * h + 1] += (double)tm0;
+                            av[2 * h + 1] += (double)tv0;
+                            am[2 * h + 2] += (double)tm1;
+                            av[2 * h + 2] += (double)tv1;
+                        }
+                        if (fbits & 1u) {  // face 0
+                            const float df = gf0 - P.z;
+                            const float sq = df * df;
+                            float dist;
+                            if (DIR == 0) dist = sq + hoist0;
+                            else if (DIR == 1) dist = hoist1 + (hoist0 + sq);
+                            else dist = hoist1 + (sq + hoist0);
+                            const float df2 = (dist + df) + 0.25f;
+                            float w = fmaxf(1.0f - df2 * inv_r2, 0.0f);
+                            w = (w * w) * w;
+                            am[0] += (double)(w * m_p);
+                            av[0] += (double)(w * scale_mom);
+                        }
                     }
+                    if (deps_pending) wait_deps();
+                    // cells of a tile have overlapping face windows: the
+                    // groups add in cell order
+                    const int si0 = su * kStride[U] + sv * kStride[V] + (cell[F] - 1) * kStride[F];
+#pragma unroll
+                    for (int g = 0; g < L::G; ++g) {
+                        __syncwarp();
+                        if (on && (L::G == 1 || grp == g)) {
+#pragma unroll
+                            for (int s = 0; s < WIN; ++s) {
+                                if (s == 0 && cell[F] == 0) continue;  // below the window
+                                const int si = si0 + s * kStride[F];
+                                st[si] += am[s];
+                                st[WW + si] += av[s];
+                            }
+                        }
+                    }
+                }
+            }
+            if (odd) {
+                // rows beyond the compact ones, particle by particle
+                if (deps_pending) wait_deps();
+#pragma unroll 1
+                for (int j = s0; j < s1; ++j) {
+                    const float4 P = wslot[j - s0], R = wslot[CAP + j - s0];
+                    const uint64_t f = (uint64_t)__float_as_uint(R.y) | ((uint64_t)__float_as_uint(R.z) << 32);
+                    const uint64_t rest = f & L::outside();
+                    if (!rest) continue;
+                    const uint32_t sub = __ffs(__ballot_sync(0xffffffffu, lane < 8 && cbeg <= j && j < cend)) - 1;
+                    const int cell[3] = {2 * tc[0] + (int)(sub & 1), 2 * tc[1] + (int)((sub >> 1) & 1), 2 * tc[2] + (int)((sub >> 2) & 1)};
+                    for (int row = lane; row < WIN * WIN; row += 32) {
+                        if (!((rest >> row) & 1u)) continue;
+                        const int su = cell[U] + row % WIN, sv = cell[V] + row / WIN;
+                        const float du = (float)(b0[U] - M + su) - P.x, dv = (float)(b0[V] - M + sv) - P.y;
+                        float hoist0 = 0.0f, hoist1 = 0.0f;
+                        if (DIR == 0) hoist0 = dv * dv + du * du;
+                        else { hoist0 = dv * dv; hoist1 = du * du; }
+#pragma unroll
+                        for (int s = 0; s < WIN; ++s) {
+                            const int sf = cell[F] + s - 1;
+                            if (sf < 0 || !((f >> (56 + s)) & 1u)) continue;
+                            const float df = (float)(b0[F] - M + sf) - P.z;
+                            const float sq = df * df;
+                            float dist;
+                            if (DIR == 0) dist = sq + hoist0;
+                            else if (DIR == 1) dist = hoist1 + (hoist0 + sq);
+                            else dist = hoist1 + (sq + hoist0);
+                            const float df2 = (dist + df) + 0.25f;
+                            float w = fmaxf(1.0f - df2 * inv_r2, 0.0f);
+                            w = (w * w) * w;
+                            const int si = su * kStride[U] + sv * kStride[V] + sf * kStride[F];
+                            st[si] += (double)(w * P.w);
+                            st[WW + si] += (double)(w * R.x);
+                        }
+                    }
+                    __syncwarp();
                 }
             }
         }
@@ -556,6 +607,40 @@ __global__ void __launch_bounds__(32 * kSplatWarps, 1) p2g_cells_kernel(SplatArg
     __syncthreads();
     double* out = a.partial + ((size_t)k_pb * 3 + DIR) * 2 * WW;
     for (int i = tid; i < 2 * WW; i += blockDim.x) out[i] = st[i];
+}
+
+template <int BSX, int M, int RW>
+__global__ void __launch_bounds__(32 * SplatShape<BSX, M>::WARPS, SplatShape<BSX, M>::CTAS) p2g_cells_kernel(SplatArgs a) {
+    constexpr int W = BSX + 2 * M, WW = W * W * W;
+    constexpr int T = BSX / 2, K = M + 1, NT = T * T * T;
+    static_assert(NT < 0xffff, "tile indices must fit 16 bits");
+    extern __shared__ double st[];       // [2][W^3]: mass, momentum; then per-warp particle slots
+    __shared__ uint32_t s_done[NT];
+    __shared__ uint16_t s_order[NT];     // tiles in colour-major order
+    __shared__ uint32_t s_next;
+    const int tid = threadIdx.x;
+    for (int i = tid; i < 2 * WW; i += blockDim.x) st[i] = 0.0;
+    for (int t = tid; t < NT; t += blockDim.x) {
+        s_done[t] = 0;
+        const int tx = t % T, ty = (t / T) % T, tz = t / (T * T);
+        const int cx = tx % K, cy = ty % K, cz = tz % K;
+        const int ci = cx + K * (cy + K * cz);
+        int base = 0;
+        for (int c = 0; c < ci; ++c) {
+            const int ox = c % K, oy = (c / K) % K, oz = c / (K * K);
+            base += ((T - ox + K - 1) / K) * ((T - oy + K - 1) / K) * ((T - oz + K - 1) / K);
+        }
+        const int ntx = (T - cx + K - 1) / K, nty = (T - cy + K - 1) / K;
+        s_order[base + (tx / K) + ntx * ((ty / K) + nty * (tz / K))] = (uint16_t)t;
+    }
+    if (tid == 0) s_next = 0;
+    __syncthreads();
+    const int k_pb = blockIdx.x / 3;
+    switch (blockIdx.x % 3) {
+        case 0: splat_cells_body<BSX, M, RW, 0>(a, k_pb, st, s_done, s_order, &s_next, NT); break;
+        case 1: splat_cells_body<BSX, M, RW, 1>(a, k_pb, st, s_done, s_order, &s_next, NT); break;
+        default: splat_cells_body<BSX, M, RW, 2>(a, k_pb, st, s_done, s_order, &s_next, NT); break;
+    }
 }
 
 // Splat for r_p = 2 (M = 2), grouped by footprint anchor.  With r_p = 2 the
@@ -590,7 +675,10 @@ template <int BSX> struct SplatR2 {
     static constexpr int NF = BSX / 2;      // anchor tiles along F
     static constexpr int NT = NA * NA * NF;
     static constexpr int NSRC = 18;         // source cells of a tile
-    static constexpr int WARPS = NT < kSplatR2Warps ? NT : kSplatR2Warps;
+    // 8^3 blocks: 100 tiles, of which about four can run at a time, so small
+    // CTAs share an SM (as in SplatShape; 4.8 M particles 4.06 -> 2.40 ms)
+    static constexpr int WARPS = BSX == 8 ? 8 : kSplatR2Warps;
+    static constexpr int CTAS = BSX == 8 ? 3 : 1;
     // particles a warp stages at once: a whole typical tile (144 at 8 per cell)
     static constexpr int CAP = 160;
     // per warp: CAP x (float4 position/mass, float momentum, u8 anchor-sorted
@@ -950,7 +1038,7 @@ __device__ __forceinline__ void splat_r2_body(const SplatArgs& a, const int k_pb
 }
 
 template <int BSX>
-__global__ void __launch_bounds__(32 * kSplatR2Warps, 1) p2g_r2_kernel(SplatArgs a) {
+__global__ void __launch_bounds__(32 * SplatR2<BSX>::WARPS, SplatR2<BSX>::CTAS) p2g_r2_kernel(SplatArgs a) {
     using S = SplatR2<BSX>;
     constexpr int WW = S::WW, NA = S::NA, NF = S::NF, NT = S::NT;
     extern __shared__ double st[];  // [2][W^3]: mass, momentum; then per-warp staging slots
@@ -1052,21 +1140,26 @@ __global__ void active_nbr_kernel(const uint64_t* active, size_t n_active, const
 
 static unsigned grid_for(size_t n) { return (unsigned)std::min<size_t>(std::max<size_t>(div_up(n, 256), 1), 8192); }
 
-template <int BSX, int M, int DIR>
-static void launch_splat_dir(msbg_ctx* ctx, const SplatArgs& a, size_t npb) {
+template <int BSX, int M, int RW>
+static void launch_splat_cells(msbg_ctx* ctx, const SplatArgs& a, size_t npb) {
+    using S = SplatShape<BSX, M>;
     constexpr int W = BSX + 2 * M;
-    constexpr int T = BSX / 2, NT = T * T * T;
-    constexpr int WARPS = NT < kSplatWarps ? NT : kSplatWarps;
-    const size_t smem = 2 * sizeof(double) * W * W * W + (size_t)WARPS * 2 * SplatCap<BSX, M>::v * sizeof(float4);
+    const size_t smem = 2 * sizeof(double) * W * W * W + (size_t)S::WARPS * 2 * S::CAP * sizeof(float4);
     static bool attr = false;
     if (!attr) {
-        CUDA_CHECK(cudaFuncSetAttribute(p2g_cells_kernel<BSX, M, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CUDA_CHECK(cudaFuncSetAttribute(p2g_cells_kernel<BSX, M, RW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr = true;
     }
     begin_launch(ctx);
-    p2g_cells_kernel<BSX, M, DIR><<<(unsigned)npb, 32 * WARPS, smem, ctx->stream>>>(a);
+    p2g_cells_kernel<BSX, M, RW><<<(unsigned)(3 * npb), 32 * S::WARPS, smem, ctx->stream>>>(a);
     after_launch(ctx, "p2g_cells_kernel");
 }
+
+// Rows along a lane axis that a footprint of radius r_p covers about its cell
+// unless a coordinate lies exactly on a cell centre: a particle at fraction f
+// of its cell reaches ceil(f - r_p - 1/2) .. floor(f + r_p - 1/2), for 0 < f < 1
+// within -floor(r_p) .. ceil(r_p - 1/2) - that is -h .. h with h = ceil(r_p - 1/2).
+static int compact_rows(float r_p) { return 2 * (int)ceilf(r_p - 0.5f) + 1; }
 
 template <int BSX, int M>
 static void launch_splat(msbg_ctx* ctx, const SplatArgs& a, size_t npb) {
@@ -1083,9 +1176,15 @@ static void launch_splat(msbg_ctx* ctx, const SplatArgs& a, size_t npb) {
         after_launch(ctx, "p2g_r2_kernel");
         return;
     }
-    launch_splat_dir<BSX, M, 0>(ctx, a, npb);
-    launch_splat_dir<BSX, M, 1>(ctx, a, npb);
-    launch_splat_dir<BSX, M, 2>(ctx, a, npb);
+    // rows beyond these are added one particle at a time, so a narrower
+    // choice is always right and only slow when many particles need it
+    if constexpr (M > 1) {
+        if (compact_rows(a.r_p) < 2 * M + 1) {
+            launch_splat_cells<BSX, M, 2 * M - 1>(ctx, a, npb);
+            return;
+        }
+    }
+    launch_splat_cells<BSX, M, 2 * M + 1>(ctx, a, npb);
 }
 
 template <int BSX, int M>
