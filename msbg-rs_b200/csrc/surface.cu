@@ -5,13 +5,15 @@
 // reconstruct_and_smooth.
 //
 // Splat on the device: particles are Morton-sorted, so each 16^3 block's
-// particles are one contiguous range ("particle blocks").  One CTA per
-// particle block stages its (bsx + 2m)^3 window (m = ceil(r_scan)) in shared
-// memory as 32-bit words (the quantised Density value, or the bits of the
-// non-negative f32 ratio, whose order is the float order) and takes the
-// minimum with shared atomics; the window's touched voxels are then committed
-// with global atomic minima into a 32-bit field over the grid's slots, which a
-// last kernel converts into the grid's payload.  A minimum does not depend on
+// particles are one contiguous range ("particle blocks").  A CTA takes a
+// particle block, or a part of its particles when there are few blocks, and
+// keeps the least squared distance of every voxel of its (bsx + 2m)^3 window
+// (m = ceil(r_scan)) in shared memory as f32 bits (non-negative, so their
+// integer order is the float order); the touched voxels are then quantised
+// and committed with global atomic minima into a 32-bit field over the grid's
+// slots, which a last kernel converts into the grid's payload.  Quantising
+// is monotone, so the minimum of the quantised values is the quantised
+// minimum.  A minimum does not depend on
 // the order of its operands, so the result is deterministic and equals the
 // crate's staged, colour-ordered commit bit for bit.
 #include <algorithm>
@@ -29,7 +31,7 @@ struct SurfArgs {
     const int32_t* dense;      // bid -> slot code, or null (hash)
     DevHash hash;
     int64_t sx, sy, sz, nx, ny;
-    int lg, m, W;
+    int lg, m, W, P;           // window extent and its row pitch
     float r_scan, dmax, inv;
     int qmax;                  // stored integer scale: 65535 Density, 255 Density8, 0 f32
     uint32_t full;
@@ -94,22 +96,49 @@ __global__ void sf_fill_kernel(uint32_t* __restrict__ f, size_t n, uint32_t v) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) f[i] = v;
 }
 
-// One CTA per particle block: stage (min in shared memory), then commit the
-// touched window voxels (global atomic min).  Each warp takes a particle; its
-// lanes take the footprint rows (iy, iz) and walk x, evaluating the crate's
+// Threads of a splat CTA, and the row pitch of its window: a warp covers 8
+// voxels along x of 4 rows, which lie on 32 different banks when the pitch is
+// 8 or 24 modulo 32.
+constexpr int kSplatThreads = 512;
+static int splat_pitch(int W) { return ((W + 7) / 16) * 16 + 8; }
+// Few particle blocks leave SMs idle: their particles are split over this
+// many CTAs at most (each commits its own window).
+constexpr int kSplatMaxParts = 32;
+
+// CTA (block, part): least squared distances in shared memory, then the commit
+// of the touched voxels (global atomic min).  Each warp takes a particle and
+// walks its footprint in tiles of 8 x 4 voxels (x, y), evaluating the crate's
 // f32 distance in its order (splat.rs:217-250: dz2 = dz dz, dyz = dz2 + dy dy,
-// dist_sq = dx dx + dyz) and quantising as channel.rs:392-417.
-__global__ void __launch_bounds__(256) sf_splat_kernel(SurfArgs a) {
+// dist_sq = dx dx + dyz).  A voxel is read first and the shared atomic issued
+// only for a smaller distance: of the hundred or so particles that reach a
+// voxel only a few lower it.  (Bound by issue: with lanes over rows, whose
+// addresses shared 4 banks, and an atomic and a quantisation per voxel, 2 M
+// particles in 256^3 took 2.76 ms on B200.)
+__global__ void __launch_bounds__(kSplatThreads) sf_splat_kernel(SurfArgs a) {
     extern __shared__ uint32_t win[];
-    const int W = a.W, WW = W * W * W, bsx = 1 << a.lg, m = a.m;
-    for (int i = threadIdx.x; i < WW; i += blockDim.x) win[i] = a.full;
+    const int W = a.W, P = a.P, WW = W * W * P, bsx = 1 << a.lg, m = a.m;
+    constexpr uint32_t kUntouched = 0x7f800000u;  // +infinity
+    const uint64_t s0 = a.pb_starts[blockIdx.x], n_all = a.pb_starts[blockIdx.x + 1] - s0;
+    const uint64_t part = (n_all + gridDim.y - 1) / gridDim.y;
+    const uint64_t s = s0 + min(n_all, part * blockIdx.y), e = s0 + min(n_all, part * (blockIdx.y + 1));
+    if (s == e) return;
+    for (int i = threadIdx.x; i < WW; i += blockDim.x) win[i] = kUntouched;
     const uint64_t key = a.pb_key[blockIdx.x];
     const int32_t b0[3] = {(int32_t)compact3(key) * bsx, (int32_t)compact3(key >> 1) * bsx, (int32_t)compact3(key >> 2) * bsx};
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const uint64_t s = a.pb_starts[blockIdx.x], e = a.pb_starts[blockIdx.x + 1];
-    for (uint64_t i = s + warp; i < e; i += nw) {
-        const float p[3] = {a.pos[3 * i], a.pos[3 * i + 1], a.pos[3 * i + 2]};
+    const int tx = lane & 7, ty = lane >> 3;
+    const float dmax = a.dmax;
+    // a contiguous range per warp: Morton neighbours share most voxels, so a
+    // warp's own earlier particles have lowered them already, and the warps
+    // work on different voxels
+    const uint64_t per = (e - s + nw - 1) / nw;
+    const uint64_t w0 = min(e, s + per * warp), w1 = min(e, w0 + per);
+    float np[3] = {0.0f, 0.0f, 0.0f};  // the next particle, one ahead
+    if (w0 < w1) { np[0] = a.pos[3 * w0]; np[1] = a.pos[3 * w0 + 1]; np[2] = a.pos[3 * w0 + 2]; }
+    for (uint64_t i = w0; i < w1; ++i) {
+        const float p[3] = {np[0], np[1], np[2]};
+        if (i + 1 < w1) { np[0] = a.pos[3 * i + 3]; np[1] = a.pos[3 * i + 4]; np[2] = a.pos[3 * i + 5]; }
         int32_t lo[3], hi[3];
 #pragma unroll
         for (int ax = 0; ax < 3; ++ax) {
@@ -117,22 +146,29 @@ __global__ void __launch_bounds__(256) sf_splat_kernel(SurfArgs a) {
             hi[ax] = min(max((int32_t)floorf((p[ax] + a.r_scan) - 0.5f), b0[ax] - m), b0[ax] + bsx + m - 1);
         }
         const float px0 = p[0] - 0.5f, py0 = p[1] - 0.5f, pz0 = p[2] - 0.5f;
-        const int ny_ = hi[1] - lo[1] + 1, nrows = ny_ * (hi[2] - lo[2] + 1);
-        for (int r = lane; r < nrows; r += 32) {
-            const int iy = lo[1] + r % ny_, iz = lo[2] + r / ny_;
-            const float dz = (float)iz - pz0;
-            const float dz2 = dz * dz;
-            const float dy = (float)iy - py0;
-            const float dyz = dz2 + dy * dy;
-            const int row = ((iz - (b0[2] - m)) * W + (iy - (b0[1] - m))) * W - (b0[0] - m);  // + ix >= 0
-            for (int ix = lo[0]; ix <= hi[0]; ++ix) {
-                const float dx = (float)ix - px0;
-                const float d2 = dx * dx + dyz;
-                if (d2 <= a.dmax) {
-                    const float t = d2 * a.inv;
-                    const uint32_t q = a.qmax ? ((uint32_t)(int32_t)roundf(t * (float)a.qmax) & (uint32_t)a.qmax)
-                                              : __float_as_uint(t);
-                    atomicMin(win + row + ix, q);
+        for (int ix = lo[0] + tx; __any_sync(0xffffffffu, ix <= hi[0]); ix += 8) {
+            const float dx = (float)ix - px0;
+            const float dx2 = ix <= hi[0] ? dx * dx : INFINITY;  // beyond the footprint: never within dmax
+            for (int iy = lo[1] + ty; __any_sync(0xffffffffu, iy <= hi[1]); iy += 4) {
+                const float dy = (float)iy - py0;
+                const float dy2 = iy <= hi[1] ? dy * dy : INFINITY;
+                // lanes beyond the footprint read the window's first row
+                const bool on = ix <= hi[0] && iy <= hi[1];
+                int at = on ? ((lo[2] - (b0[2] - m)) * W + (iy - (b0[1] - m))) * P + ix - (b0[0] - m) : 0;
+                const int step = on ? W * P : 0;
+                for (int iz = lo[2]; iz <= hi[2]; iz += 4, at += 4 * step) {
+                    // four loads in flight, then the compares
+                    uint32_t cur[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) cur[u] = iz + u <= hi[2] ? *(volatile uint32_t*)(win + at + u * step) : 0u;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float dz = (float)(iz + u) - pz0;
+                        const float dz2 = dz * dz;
+                        const float dyz = dz2 + dy2;
+                        const float d2 = dx2 + dyz;
+                        if (d2 <= dmax && __float_as_uint(d2) < cur[u]) atomicMin(win + at + u * step, __float_as_uint(d2));
+                    }
                 }
             }
         }
@@ -140,9 +176,10 @@ __global__ void __launch_bounds__(256) sf_splat_kernel(SurfArgs a) {
     __syncthreads();
     const int N = bsx * bsx * bsx, msk = bsx - 1;
     for (int i = threadIdx.x; i < WW; i += blockDim.x) {
-        const uint32_t v = win[i];
-        if (v == a.full) continue;
-        const int64_t gx = b0[0] - m + i % W, gy = b0[1] - m + (i / W) % W, gz = b0[2] - m + i / (W * W);
+        if (win[i] == kUntouched) continue;
+        const float t = __uint_as_float(win[i]) * a.inv;
+        const uint32_t v = a.qmax ? ((uint32_t)(int32_t)roundf(t * (float)a.qmax) & (uint32_t)a.qmax) : __float_as_uint(t);
+        const int64_t gx = b0[0] - m + i % P, gy = b0[1] - m + (i / P) % W, gz = b0[2] - m + i / (W * P);
         if (gx < 0 || gy < 0 || gz < 0 || gx >= a.sx || gy >= a.sy || gz >= a.sz) continue;
         const int32_t code = surf_code(a, (uint64_t)(gx >> a.lg) + (uint64_t)(gy >> a.lg) * a.nx +
                                               (uint64_t)(gz >> a.lg) * a.nx * a.ny);
@@ -342,16 +379,19 @@ static std::vector<uint64_t> surface_splat(msbg_grid* g, const float* d_pos, siz
     a.hash = device_hash(g);
     a.sx = (int64_t)g->sx; a.sy = (int64_t)g->sy; a.sz = (int64_t)g->sz;
     a.nx = (int64_t)g->nx; a.ny = (int64_t)g->ny;
-    a.lg = lg; a.m = m; a.W = W;
+    a.lg = lg; a.m = m; a.W = W; a.P = splat_pitch(W);
     a.r_scan = r_scan;
     a.dmax = r_scan * r_scan;
     a.inv = 1.0f / a.dmax;
     a.qmax = qmax;
     a.full = full;
-    const size_t smem = (size_t)W * W * W * 4;
+    const size_t smem = (size_t)W * W * a.P * 4;
     CUDA_CHECK(cudaFuncSetAttribute(sf_splat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // about two CTAs for each of an SM's four places, and at least 1,024
+    // particles a CTA on average: fewer do not pay for another window
+    const size_t parts = std::min<size_t>({div_up(148 * 8, npb), std::max<size_t>(n / (npb * 1024), 1), kSplatMaxParts});
     begin_launch(ctx);
-    sf_splat_kernel<<<(unsigned)npb, 256, smem, ctx->stream>>>(a);
+    sf_splat_kernel<<<dim3((unsigned)npb, (unsigned)parts), kSplatThreads, smem, ctx->stream>>>(a);
     after_launch(ctx, "sf_splat_kernel");
     if (!active.empty()) {
         begin_launch(ctx);
