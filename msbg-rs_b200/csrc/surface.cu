@@ -17,6 +17,7 @@
 // the order of its operands, so the result is deterministic and equals the
 // crate's staged, colour-ordered commit bit for bit.
 #include <algorithm>
+#include <type_traits>
 
 #include "grid.cuh"
 #include "sort.cuh"
@@ -106,77 +107,109 @@ static int splat_pitch(int W) { return ((W + 7) / 16) * 16 + 8; }
 constexpr int kSplatMaxParts = 32;
 
 // CTA (block, part): least squared distances in shared memory, then the commit
-// of the touched voxels (global atomic min).  Each warp takes a particle and
-// walks its footprint in tiles of 8 x 4 voxels (x, y), evaluating the crate's
-// f32 distance in its order (splat.rs:217-250: dz2 = dz dz, dyz = dz2 + dy dy,
-// dist_sq = dx dx + dyz).  A voxel is read first and the shared atomic issued
-// only for a smaller distance: of the hundred or so particles that reach a
-// voxel only a few lower it.  (Bound by issue: with lanes over rows, whose
-// addresses shared 4 banks, and an atomic and a quantisation per voxel, 2 M
-// particles in 256^3 took 2.76 ms on B200.)
+// of the touched voxels (global atomic min).  Each lane prepares one of 32
+// particles (its clipped footprint, window coordinates in 6 bits each), then
+// the warp takes them in turn, broadcast by shuffles: its lanes cover 8 x 4
+// voxels (x, y), twice along y, and walk z, evaluating the crate's f32
+// distance in its order (splat.rs:217-250: dz2 = dz dz, dyz = dz2 + dy dy,
+// dist_sq = dx dx + dyz).  Coordinates past the footprint's end repeat its last
+// voxel, which a minimum does not mind.  A voxel is read first and the shared
+// atomic issued only for a smaller distance: of the hundred or so particles
+// that reach a voxel only a few lower it; untouched voxels hold the word
+// above dmax's, so the same comparison is the radius test.
+// Bound by issue.  2 M particles in 256^3, r_scan 4 (B200): 2.76 ms with lanes
+// over rows, whose addresses shared 4 banks, and an atomic and a quantisation
+// per voxel; 1.02 ms with this tiling and every lane preparing every particle
+// (431 warp instructions per particle); 0.66 ms as it stands.
 __global__ void __launch_bounds__(kSplatThreads) sf_splat_kernel(SurfArgs a) {
     extern __shared__ uint32_t win[];
     const int W = a.W, P = a.P, WW = W * W * P, bsx = 1 << a.lg, m = a.m;
-    constexpr uint32_t kUntouched = 0x7f800000u;  // +infinity
+    const uint32_t untouched = __float_as_uint(a.dmax) + 1u;
     const uint64_t s0 = a.pb_starts[blockIdx.x], n_all = a.pb_starts[blockIdx.x + 1] - s0;
     const uint64_t part = (n_all + gridDim.y - 1) / gridDim.y;
     const uint64_t s = s0 + min(n_all, part * blockIdx.y), e = s0 + min(n_all, part * (blockIdx.y + 1));
     if (s == e) return;
-    for (int i = threadIdx.x; i < WW; i += blockDim.x) win[i] = kUntouched;
+    for (int i = threadIdx.x; i < WW; i += blockDim.x) win[i] = untouched;
     const uint64_t key = a.pb_key[blockIdx.x];
     const int32_t b0[3] = {(int32_t)compact3(key) * bsx, (int32_t)compact3(key >> 1) * bsx, (int32_t)compact3(key >> 2) * bsx};
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int tx = lane & 7, ty = lane >> 3;
-    const float dmax = a.dmax;
+    const int zstep = W * P;
+    // the window's first coordinates (below 2^21 + bsx: exact in f32, as is
+    // every coordinate formed from them)
+    const float g0 = (float)(b0[0] - m), g1 = (float)(b0[1] - m), g2 = (float)(b0[2] - m);
     // a contiguous range per warp: Morton neighbours share most voxels, so a
     // warp's own earlier particles have lowered them already, and the warps
     // work on different voxels
     const uint64_t per = (e - s + nw - 1) / nw;
     const uint64_t w0 = min(e, s + per * warp), w1 = min(e, w0 + per);
-    float np[3] = {0.0f, 0.0f, 0.0f};  // the next particle, one ahead
-    if (w0 < w1) { np[0] = a.pos[3 * w0]; np[1] = a.pos[3 * w0 + 1]; np[2] = a.pos[3 * w0 + 2]; }
-    for (uint64_t i = w0; i < w1; ++i) {
-        const float p[3] = {np[0], np[1], np[2]};
-        if (i + 1 < w1) { np[0] = a.pos[3 * i + 3]; np[1] = a.pos[3 * i + 4]; np[2] = a.pos[3 * i + 5]; }
-        int32_t lo[3], hi[3];
+    for (uint64_t i0 = w0; i0 < w1; i0 += 32) {
+        float q[3] = {0.0f, 0.0f, 0.0f};
+        uint32_t lo = 0, hi = 0;  // window coordinates, 6 bits per axis
+        bool any = false;
+        if (i0 + lane < w1) {
+            any = true;
 #pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            lo[ax] = min(max((int32_t)ceilf((p[ax] - a.r_scan) - 0.5f), b0[ax] - m), b0[ax] + bsx + m - 1);
-            hi[ax] = min(max((int32_t)floorf((p[ax] + a.r_scan) - 0.5f), b0[ax] - m), b0[ax] + bsx + m - 1);
+            for (int ax = 0; ax < 3; ++ax) {
+                const float p = a.pos[3 * (i0 + lane) + ax];
+                const int32_t l = min(max((int32_t)ceilf((p - a.r_scan) - 0.5f), b0[ax] - m), b0[ax] + bsx + m - 1) - (b0[ax] - m);
+                const int32_t h = min(max((int32_t)floorf((p + a.r_scan) - 0.5f), b0[ax] - m), b0[ax] + bsx + m - 1) - (b0[ax] - m);
+                any = any && l <= h;
+                lo |= (uint32_t)l << (6 * ax);
+                hi |= (uint32_t)h << (6 * ax);
+                q[ax] = p - 0.5f;
+            }
         }
-        const float px0 = p[0] - 0.5f, py0 = p[1] - 0.5f, pz0 = p[2] - 0.5f;
-        for (int ix = lo[0] + tx; __any_sync(0xffffffffu, ix <= hi[0]); ix += 8) {
-            const float dx = (float)ix - px0;
-            const float dx2 = ix <= hi[0] ? dx * dx : INFINITY;  // beyond the footprint: never within dmax
-            for (int iy = lo[1] + ty; __any_sync(0xffffffffu, iy <= hi[1]); iy += 4) {
-                const float dy = (float)iy - py0;
-                const float dy2 = iy <= hi[1] ? dy * dy : INFINITY;
-                // lanes beyond the footprint read the window's first row
-                const bool on = ix <= hi[0] && iy <= hi[1];
-                int at = on ? ((lo[2] - (b0[2] - m)) * W + (iy - (b0[1] - m))) * P + ix - (b0[0] - m) : 0;
-                const int step = on ? W * P : 0;
-                for (int iz = lo[2]; iz <= hi[2]; iz += 4, at += 4 * step) {
-                    // four loads in flight, then the compares
-                    uint32_t cur[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) cur[u] = iz + u <= hi[2] ? *(volatile uint32_t*)(win + at + u * step) : 0u;
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float dz = (float)(iz + u) - pz0;
-                        const float dz2 = dz * dz;
-                        const float dyz = dz2 + dy2;
-                        const float d2 = dx2 + dyz;
-                        if (d2 <= dmax && __float_as_uint(d2) < cur[u]) atomicMin(win + at + u * step, __float_as_uint(d2));
+        for (uint32_t live = __ballot_sync(0xffffffffu, any); live; live &= live - 1) {
+            const int src = __ffs(live) - 1;
+            const float px0 = __shfl_sync(0xffffffffu, q[0], src), py0 = __shfl_sync(0xffffffffu, q[1], src),
+                        pz0 = __shfl_sync(0xffffffffu, q[2], src);
+            const uint32_t l = __shfl_sync(0xffffffffu, lo, src), h = __shfl_sync(0xffffffffu, hi, src);
+            const int x0 = l & 63, y0 = (l >> 6) & 63, z0 = l >> 12, x1 = h & 63, y1 = (h >> 6) & 63, nz = (int)(h >> 12) - z0 + 1;
+            const float dz_first = g2 + (float)z0;
+            for (int xx = x0; xx <= x1; xx += 8) {
+                const int ix = min(xx + tx, x1);
+                const float dx = (g0 + (float)ix) - px0, dx2 = dx * dx;
+                // TWO: the rows of a second tile, 4 further along y
+                auto tiles = [&](int yy, auto two) {
+                    constexpr bool TWO = decltype(two)::value;
+                    const int iy = min(yy + ty, y1), jy = TWO ? min(yy + ty + 4, y1) : iy;
+                    const float dy = (g1 + (float)iy) - py0, dy2 = dy * dy;
+                    const float ey = (g1 + (float)jy) - py0, ey2 = ey * ey;
+                    uint32_t* pa = win + (z0 * W + iy) * P + ix;
+                    const int off = TWO ? (jy - iy) * P : 0;
+                    float fz = dz_first;
+                    for (int z = 0; z < nz; z += 2) {
+                        const bool last = z + 1 >= nz;  // the second plane repeats the first
+                        uint32_t* pb = last ? pa : pa + zstep;
+                        const uint32_t ca = *(volatile uint32_t*)pa, cb = *(volatile uint32_t*)pb;
+                        uint32_t da = 0, db = 0;
+                        if (TWO) { da = *(volatile uint32_t*)(pa + off); db = *(volatile uint32_t*)(pb + off); }
+                        const float dza = fz - pz0, dzb = (last ? fz : fz + 1.0f) - pz0;
+                        const float za2 = dza * dza, zb2 = dzb * dzb;
+                        const uint32_t va = __float_as_uint(dx2 + (za2 + dy2)), vb = __float_as_uint(dx2 + (zb2 + dy2));
+                        if (va < ca) atomicMin(pa, va);
+                        if (vb < cb) atomicMin(pb, vb);
+                        if (TWO) {
+                            const uint32_t wa = __float_as_uint(dx2 + (za2 + ey2)), wb = __float_as_uint(dx2 + (zb2 + ey2));
+                            if (wa < da) atomicMin(pa + off, wa);
+                            if (wb < db) atomicMin(pb + off, wb);
+                        }
+                        pa += 2 * zstep;
+                        fz += 2.0f;
                     }
-                }
+                };
+                int yy = y0;
+                for (; yy + 4 <= y1; yy += 8) tiles(yy, std::true_type());
+                if (yy <= y1) tiles(yy, std::false_type());
             }
         }
     }
     __syncthreads();
     const int N = bsx * bsx * bsx, msk = bsx - 1;
     for (int i = threadIdx.x; i < WW; i += blockDim.x) {
-        if (win[i] == kUntouched) continue;
+        if (win[i] == untouched) continue;
         const float t = __uint_as_float(win[i]) * a.inv;
         const uint32_t v = a.qmax ? ((uint32_t)(int32_t)roundf(t * (float)a.qmax) & (uint32_t)a.qmax) : __float_as_uint(t);
         const int64_t gx = b0[0] - m + i % P, gy = b0[1] - m + (i / P) % W, gz = b0[2] - m + i / (W * P);
