@@ -134,6 +134,37 @@ struct ScratchLayout {
 // stream first, so kernels still in flight never see their scratch freed.
 char* scratch(msbg_ctx* ctx, const ScratchLayout& L);
 
+// Programmatic dependent launch: a kernel launched with launch_chained may be
+// scheduled as soon as every CTA of the kernel before it on the stream has
+// called chain_trigger (or ended); before its first access to data that
+// kernels in flight write it calls chain_wait, which returns when the kernel
+// before it has finished with all its writes visible (and that one, having
+// waited itself, after every earlier one).  Launch latency, CTA start-up and
+// reads of data no kernel in flight writes then overlap the kernel before.
+// Data read after chain_wait must not come through `const __restrict__`
+// pointers: those reads may be moved ahead of it.
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// cluster > 1: thread-block clusters of that many CTAs along x.
+template <class... P, class... A>
+inline void launch_chained(cudaStream_t stream, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // Nanoseconds of the GPU's global timer (bounded waits measure with it).
 __device__ __forceinline__ uint64_t globaltimer_ns() {
     uint64_t t;

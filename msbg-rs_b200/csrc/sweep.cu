@@ -381,8 +381,8 @@ __device__ __forceinline__ void stage_general(const SweepArgs& a, float* __restr
 }
 
 template <class E, int BSX, int ST>
-__global__ void __launch_bounds__(BSX * BSX < 32 ? 32 : BSX * BSX, BSX == 16 && ST == MSBG_BILAPLACIAN ? 4 : 1)
-sweep_phase_kernel(SweepArgs a, const int32_t* __restrict__ order, int n) {
+__global__ void __launch_bounds__(BSX * BSX < 32 ? 32 : BSX * BSX, BSX == 16 ? 4 : BSX == 8 ? 12 : 1)
+sweep_phase_kernel(SweepArgs a, const int32_t* __restrict__ order) {
     constexpr int HALO = ST == MSBG_BILAPLACIAN ? 2 : 1;
     constexpr int HSX = BSX + 2 * HALO;
     constexpr int RS = Stage<BSX>::RS;
@@ -398,15 +398,17 @@ sweep_phase_kernel(SweepArgs a, const int32_t* __restrict__ order, int n) {
     typename E::T* payload = (typename E::T*)a.payload;
     const int tid = threadIdx.x, nthr = blockDim.x;
 
-    for (int t = blockIdx.x; t < n; t += gridDim.x) {
+    chain_trigger();
+    {
+        const int t = blockIdx.x;  // one block per CTA
         const int pi = order[t];
-        __syncthreads();  // the previous block's compute is done with h
         if (tid < 27) nb[tid] = a.nbr[(size_t)pi * 27 + tid];
         if (tid == 32 || (nthr <= 32 && tid == 31)) {
             flags = a.bxyz[(size_t)pi * 8 + 3];
             sides = a.bxyz[(size_t)pi * 8 + 4];
         }
         __syncthreads();
+        chain_wait();  // the plan's tables are read already: they belong to no kernel
         if (staged_by_planes<HALO>(flags)) {
             // Fast path: the block's needed halo lies inside the domain or
             // mirrors whole planes of its own layer, so every staged cell
@@ -1064,6 +1066,7 @@ sweep_compact_kernel(SweepArgs a, const int32_t* __restrict__ order, int n) {
         }
     };
     int pi2 = 0;
+    chain_trigger();
     if (meta_thread) {
         int32_t nbv = 0, mv = 0;
         const int pi0 = order[t];
@@ -1077,6 +1080,7 @@ sweep_compact_kernel(SweepArgs a, const int32_t* __restrict__ order, int n) {
         if (t + 2 * g < n) pi2 = order[t + 2 * g];
     }
     __syncthreads();
+    chain_wait();  // the plan's tables are read already: they belong to no kernel
     constexpr int NT = CompactThreads<BSX, ST, PAIR>::v;
     if (staged_by_planes<1>(flg[0])) issue_compact<BSX, ST, NT>(a, hb, nbs[0], flg[0], mirs[0]);
     cp_async_commit();
@@ -1331,6 +1335,7 @@ __global__ void __launch_bounds__(BSX * BSX) sweep_cluster_kernel(SweepArgs a, c
     __shared__ int32_t tab[3 * (BSX + 2)];
     const int tid = threadIdx.x;
     const int t = blockIdx.x / NS, z0 = (int)(blockIdx.x % NS) * ZS;
+    chain_trigger();
     const int pi = order[t];
     if (tid < 27) nbs[tid] = a.nbr[(size_t)pi * 27 + tid];
     if (tid == BSX * BSX - 1) {
@@ -1338,6 +1343,7 @@ __global__ void __launch_bounds__(BSX * BSX) sweep_cluster_kernel(SweepArgs a, c
         mirs = a.bxyz[(size_t)pi * 8 + 4];
     }
     __syncthreads();
+    chain_wait();
     if (staged_by_planes<1>(flg)) {
         issue_compact<BSX, ST, BSX * BSX, false, true>(a, hb, nbs, flg, mirs, z0, z0 + ZS + 1);
         cp_async_commit();
@@ -1364,20 +1370,9 @@ static void launch_cluster(msbg_ctx* ctx, const SweepArgs& a, const int32_t* ord
                                         (int)smem));
         attr = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n * NS));
-    cfg.blockDim = dim3(BSX * BSX);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = NS;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
     begin_launch(ctx);
-    CUDA_CHECK(cudaLaunchKernelEx(&cfg, sweep_cluster_kernel<BSX, ST, CLAMP, ZS>, a, order, n));
+    launch_chained(ctx->stream, sweep_cluster_kernel<BSX, ST, CLAMP, ZS>, dim3((unsigned)(n * NS)), dim3(BSX * BSX), smem, NS, a,
+                   order, n);
     after_launch(ctx, "sweep_cluster_kernel");
 }
 
@@ -1399,7 +1394,8 @@ static void launch_compact_v(msbg_ctx* ctx, const SweepArgs& a, const int32_t* o
     CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     const int grid = std::max(1, std::min(n, std::max(per_sm, 1) * sms));
     begin_launch(ctx);
-    sweep_compact_kernel<BSX, ST, CLAMP, PAIR><<<(unsigned)grid, threads, smem, ctx->stream>>>(a, order, n);
+    launch_chained(ctx->stream, sweep_compact_kernel<BSX, ST, CLAMP, PAIR>, dim3((unsigned)grid), dim3((unsigned)threads), smem, 1,
+                   a, order, n);
     after_launch(ctx, "sweep_compact_kernel");
 }
 
@@ -1514,7 +1510,7 @@ static void launch_phase(msbg_ctx* ctx, const SweepArgs& a, const int32_t* order
         return;
     }
     begin_launch(ctx);
-    sweep_phase_kernel<E, BSX, ST><<<(unsigned)n, threads, smem, ctx->stream>>>(a, order, n);
+    launch_chained(ctx->stream, sweep_phase_kernel<E, BSX, ST>, dim3((unsigned)n), dim3((unsigned)threads), smem, 1, a, order);
     after_launch(ctx, "sweep_phase_kernel");
 }
 
