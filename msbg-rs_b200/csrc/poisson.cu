@@ -98,7 +98,7 @@ struct msbg_poisson {
     // while loop, no host read between them), one per (method, b, x64).
     struct SGraph {
         int method;
-        const float* b;
+        const float* b;  // method 0 (method 1's loop does not read it: null)
         const double* x64;
         cudaGraphExec_t exec;
         int kernels_first, kernels_body;  // launches before the loop and per loop iteration
@@ -106,6 +106,7 @@ struct msbg_poisson {
     std::vector<SGraph> sgraphs;
     msbg::DevBuf sctl;   // SolveCtl of the captured loops
     msbg::DevBuf shist;  // f64 [capacity] relative residual per iteration
+    msbg::DevBuf dpart;  // f64 [kFusedDotMax] partials of the fused dot products, then their ticket
     ~msbg_poisson() {
         for (auto& g : vgraphs)
             if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -331,28 +332,136 @@ __global__ void __launch_bounds__(256) pk_block16(LevelArgs L, const float* __re
     }
 }
 
-// Quad tile: one 64-thread CTA per block; thread (q, y) owns the four
-// x-consecutive cells 4q..4q+3 of row y and walks all 16 z-planes with the
+// ---- dot products inside the kernels that produce their operands ------------
+// CG scalars kept on the device between kernels (one host read per iteration):
+// sc[SC_RZ] = r.z, sc[SC_PQ] = p.Ap, sc[SC_ALPHA], sc[SC_RR] = r.r,
+// sc[SC_RZ2] = the new r.z, sc[SC_ZR] = z.r_old (flexible CG), sc[SC_BETA],
+// sc[SC_BAD] != 0 when p.Ap <= 0 or r.z is not finite (the updates below are
+// then skipped and the host restarts or stops).
+enum { SC_RZ, SC_PQ, SC_ALPHA, SC_RR, SC_RZ2, SC_ZR, SC_BETA, SC_BAD, SC_COUNT };
+
+// Control block of a captured solve loop: iterations run, the limit, the
+// stopping threshold tol |b| and |b|.
+struct SolveCtl {
+    long long it, max_iter;
+    double thr, bn;
+};
+
+__device__ __forceinline__ void cg_alpha(double* sc, double pq) {
+    const double rz = sc[SC_RZ];
+    const bool bad = !(pq > 0.0) || !isfinite(rz);
+    sc[SC_PQ] = pq;
+    sc[SC_BAD] = bad ? 1.0 : 0.0;
+    sc[SC_ALPHA] = bad ? 0.0 : rz / pq;
+}
+// beta = r.z_new / r.z (or (r.z_new - z.r_old) / r.z for flexible CG); r.z = r.z_new.
+__device__ __forceinline__ void cg_beta(double* sc, int flexible) {
+    const double rz2 = sc[SC_RZ2];
+    sc[SC_BETA] = flexible ? (rz2 - sc[SC_ZR]) / sc[SC_RZ] : rz2 / sc[SC_RZ];
+    sc[SC_RZ] = rz2;
+}
+// The test at the end of a captured solve iteration: counts it, records
+// |r| / |b| and keeps the loop running while |r| > tol |b|, the limit is not
+// reached and (check_bad) CG saw no breakdown.
+__device__ __forceinline__ void solve_test(cudaGraphConditionalHandle h, const double* sc, SolveCtl* c, double* hist, int check_bad) {
+    const long long it = c->it + 1;
+    c->it = it;
+    const double rn = sqrt(sc[SC_RR]);
+    hist[it - 1] = rn / c->bn;
+    const bool bad = check_bad && sc[SC_BAD] != 0.0;
+    cudaGraphSetConditional(h, (rn > c->thr && it < c->max_iter && !bad) ? 1u : 0u);
+}
+
+// A dot product formed by the CTAs of a kernel: each writes one FP64 partial
+// and the last to finish adds them in CTA order of a fixed tree (the order
+// does not depend on which CTA that is) and runs the scalar step that needs
+// the sum.  Two launches per dot product and a pass over its operands less
+// than partial and final sums as kernels of their own.
+enum { DOT_NONE, DOT_PQ, DOT_RZ, DOT_RZ2, DOT_RR };
+struct DotArgs {
+    double* partial;      // [gridDim.x]
+    unsigned int* ticket; // 0 between kernels
+    double* sc;           // CG scalars
+    int kind;             // DOT_*
+    // DOT_RR: the solve loop's test
+    cudaGraphConditionalHandle cond;
+    SolveCtl* ctl;
+    double* hist;
+};
+// Partials of one fused dot product at most: the last CTA adds them alone.
+constexpr int64_t kFusedDotMax = 8192;
+
+template <int NT>
+__device__ __forceinline__ double cta_sum(double s, double* sm) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < NT / 32; ++w) t += sm[w];
+    return t;  // valid in thread 0
+}
+
+template <int NT>
+__device__ __forceinline__ void dot_finish(double s, const DotArgs& d) {
+    __shared__ double sm[NT / 32];
+    __shared__ bool last;
+    const double t = cta_sum<NT>(s, sm);
+    if (threadIdx.x == 0) {
+        d.partial[blockIdx.x] = t;
+        __threadfence();
+        last = atomicAdd(d.ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double v = 0.0;
+#pragma unroll 8
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += NT) v += __ldcg(d.partial + i);
+    __syncthreads();
+    const double sum = cta_sum<NT>(v, sm);
+    if (threadIdx.x == 0) {
+        *d.ticket = 0u;
+        if (d.kind == DOT_PQ) cg_alpha(d.sc, sum);
+        else if (d.kind == DOT_RZ) d.sc[SC_RZ] = sum;
+        else if (d.kind == DOT_RZ2) {
+            d.sc[SC_RZ2] = sum;
+            cg_beta(d.sc, 0);
+        } else {
+            d.sc[SC_RR] = sum;
+            solve_test(d.cond, d.sc, d.ctl, d.hist, 1);
+        }
+    }
+}
+
+// Quad tile: one 64-thread CTA per ZS z-planes of a block; thread (q, y) owns
+// the four x-consecutive cells 4q..4q+3 of row y and walks the z-planes with the
 // planes below and above in registers as float4 (plane z+2 loaded one step
 // ahead), so each thread keeps two 16-byte loads in flight per plane.  The x
 // neighbours come from the adjacent lanes of the row (shuffles) and, at the
 // block's x faces, from the neighbour blocks; the y neighbours from a
 // double-buffered shared plane whose halo rows the first and last row load
-// from the y neighbour blocks.
+// from the y neighbour blocks.  Bound by latency when the set is small: with
+// all 16 planes in a CTA, 776 blocks are 10 warps per SM; with 4 the Jacobi
+// sweep takes 8.4 instead of 12.5 us (B200).
+// DOT: x . out (OP 2) or b . out (OP 0) formed on the way (dot_finish).
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float comp(const float4& v, int e) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; }
 
-template <int OP>
+template <int OP, int ZS, bool DOT = false>
 __global__ void __launch_bounds__(64) pk_quad16(LevelArgs L, const float* __restrict__ x, const float* __restrict__ b,
-                                                float* __restrict__ out, float omega) {
+                                                float* __restrict__ out, float omega, DotArgs dot) {
     __shared__ float4 pl[2][18][4];  // rows y = -1..16 of a plane, four quads each
-    const int64_t k = blockIdx.x;
+    const int64_t k = blockIdx.x / (16 / ZS);
+    const int z0 = (int)(blockIdx.x % (16 / ZS)) * ZS;
+    double dsum = 0.0;
     const int q = threadIdx.x & 3, y = threadIdx.x >> 2;
     const int64_t base = k << 12;
     const int off = (y << 4) + (q << 2);
     const float inv_d = 1.0f / (6.0f * L.scale);
     if (OP == 0 && !x) {
-        for (int z = 0; z < 16; ++z) {
+        for (int z = z0; z < z0 + ZS; ++z) {
             const float4 bv = ld4(b + base + off + (z << 8));
             *reinterpret_cast<float4*>(out + base + off + (z << 8)) =
                 make_float4(__fmul_rn(__fmul_rn(omega, bv.x), inv_d), __fmul_rn(__fmul_rn(omega, bv.y), inv_d),
@@ -375,8 +484,9 @@ __global__ void __launch_bounds__(64) pk_quad16(LevelArgs L, const float* __rest
         if (z > 15) return nzp >= 0 ? xv4(x + ((int64_t)nzp << 12) + off) : zero;
         return xv4(x + base + off + (z << 8));
     };
-    float4 down = plane(-1), cur = plane(0), up = plane(1);
-    for (int z = 0; z < 16; ++z) {
+    float4 down = plane(z0 - 1), cur = plane(z0), up = plane(z0 + 1);
+#pragma unroll 4
+    for (int z = z0; z < z0 + ZS; ++z) {
         const int buf = z & 1;
         const float4 upn = z + 2 <= 16 ? plane(z + 2) : zero;
         const float4 bz = OP == 2 ? zero : ld4(b + base + off + (z << 8));
@@ -397,12 +507,14 @@ __global__ void __launch_bounds__(64) pk_quad16(LevelArgs L, const float* __rest
             const float xm = e == 0 ? lw : comp(cur, e - 1), xp = e == 3 ? rx : comp(cur, e + 1);
             const float sn = nb6(xm, xp, comp(ym, e), comp(yp, e), comp(down, e), comp(up, e));
             r[e] = op7<OP>(sn, comp(cur, e), comp(bz, e), L.scale, omega, inv_d);
+            if (DOT) dsum += (double)(OP == 2 ? comp(cur, e) : comp(bz, e)) * (double)r[e];
         }
         *reinterpret_cast<float4*>(out + base + off + (z << 8)) = make_float4(r[0], r[1], r[2], r[3]);
         down = cur;
         cur = up;
         up = upn;
     }
+    if (DOT) dot_finish<64>(dsum, dot);
 }
 
 // Cell-centred trilinear transfer weights along one axis: a fine cell takes
@@ -642,13 +754,6 @@ __global__ void pk_axpby(int64_t n, float a, const float* __restrict__ x, float 
         y[i] = a * x[i] + b * y[i];
 }
 
-// CG scalars kept on the device between kernels (one host read per iteration):
-// sc[SC_RZ] = r.z, sc[SC_PQ] = p.Ap, sc[SC_ALPHA], sc[SC_RR] = r.r,
-// sc[SC_RZ2] = the new r.z, sc[SC_ZR] = z.r_old (flexible CG), sc[SC_BETA],
-// sc[SC_BAD] != 0 when p.Ap <= 0 or r.z is not finite (the updates below are
-// then skipped and the host restarts or stops).
-enum { SC_RZ, SC_PQ, SC_ALPHA, SC_RR, SC_RZ2, SC_ZR, SC_BETA, SC_BAD, SC_COUNT };
-
 // Stage 2 of p.Ap (the same tree as pk_dot_final), then alpha = r.z / p.Ap.
 __global__ void __launch_bounds__(DOT_THREADS) pk_dot_final_alpha(const double* __restrict__ partial, int np,
                                                                    double* __restrict__ sc) {
@@ -661,34 +766,33 @@ __global__ void __launch_bounds__(DOT_THREADS) pk_dot_final_alpha(const double* 
         if (threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        const double pq = sm[0], rz = sc[SC_RZ];
-        const bool bad = !(pq > 0.0) || !isfinite(rz);
-        sc[SC_PQ] = pq;
-        sc[SC_BAD] = bad ? 1.0 : 0.0;
-        sc[SC_ALPHA] = bad ? 0.0 : rz / pq;
-    }
+    if (threadIdx.x == 0) cg_alpha(sc, sm[0]);
 }
 
 // x += alpha p (FP64) and r = (-alpha) q + r (f32) as fused multiply-adds,
-// skipped on breakdown.
-__global__ void pk_cg_update(int64_t n, const double* __restrict__ sc, const float* __restrict__ p,
-                             const float* __restrict__ q, double* __restrict__ x, float* __restrict__ r) {
-    if (sc[SC_BAD] != 0.0) return;
+// skipped on breakdown.  DOT: r.r of the new residual and the loop's test.
+template <bool DOT>
+__global__ void __launch_bounds__(256) pk_cg_update(int64_t n, const double* __restrict__ sc, const float* __restrict__ p,
+                                                    const float* __restrict__ q, double* __restrict__ x, float* __restrict__ r,
+                                                    DotArgs dot) {
+    const bool bad = sc[SC_BAD] != 0.0;
+    if (!DOT && bad) return;
     const double a = sc[SC_ALPHA];
     const float na = (float)-a;
+    double s = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        x[i] = fma(a, (double)p[i], x[i]);
-        r[i] = fmaf(na, q[i], r[i]);
+        float ri = r[i];
+        if (!bad) {
+            x[i] = fma(a, (double)p[i], x[i]);
+            ri = fmaf(na, q[i], ri);
+            r[i] = ri;
+        }
+        if (DOT) s += (double)ri * (double)ri;
     }
+    if (DOT) dot_finish<256>(s, dot);
 }
 
-// beta = r.z_new / r.z (or (r.z_new - z.r_old) / r.z for flexible CG); r.z = r.z_new.
-__global__ void pk_cg_beta(double* __restrict__ sc, int flexible) {
-    const double rz2 = sc[SC_RZ2];
-    sc[SC_BETA] = flexible ? (rz2 - sc[SC_ZR]) / sc[SC_RZ] : rz2 / sc[SC_RZ];
-    sc[SC_RZ] = rz2;
-}
+__global__ void pk_cg_beta(double* __restrict__ sc, int flexible) { cg_beta(sc, flexible); }
 
 // p = z + beta p (f32; beta from the device; the product rounded, then the sum)
 __global__ void pk_cg_direction(int64_t n, const double* __restrict__ sc, const float* __restrict__ z,
@@ -718,24 +822,9 @@ static LevelArgs level_args(const PLevelDev& L) {
     return LevelArgs{L.nbr.as<int32_t>(), L.lg, L.cells(), L.scale, L.diag.p ? L.diag.as<float>() : nullptr};
 }
 
-// Control block of a captured solve loop: iterations run, the limit, the
-// stopping threshold tol |b| and |b|.
-struct SolveCtl {
-    long long it, max_iter;
-    double thr, bn;
-};
-
-// The test at the end of a captured solve iteration: counts it, records
-// |r| / |b| and keeps the loop running while |r| > tol |b|, the limit is not
-// reached and (check_bad) CG saw no breakdown.  One thread.
 __global__ void pk_solve_test(cudaGraphConditionalHandle h, const double* __restrict__ sc, SolveCtl* __restrict__ c,
                               double* __restrict__ hist, int check_bad) {
-    const long long it = c->it + 1;
-    c->it = it;
-    const double rn = sqrt(sc[SC_RR]);
-    hist[it - 1] = rn / c->bn;
-    const bool bad = check_bad && sc[SC_BAD] != 0.0;
-    cudaGraphSetConditional(h, (rn > c->thr && it < c->max_iter && !bad) ? 1u : 0u);
+    solve_test(h, sc, c, hist, check_bad);
 }
 
 static void upload(msbg_ctx* ctx, DevBuf& d, const void* h, size_t bytes) {
@@ -947,17 +1036,33 @@ static void build(msbg_poisson* P, uint64_t sx, uint64_t sy, uint64_t sz, int bs
     upload(ctx, P->ainv, inv.data(), inv.size() * 8);
     const int64_t n0 = P->lv[0].cells();
     P->work.reserve((size_t)n0 * (7 * 4 + 8) + (DOT_BLOCKS + 16) * 8 + 1024);
+    P->dpart.reserve(kFusedDotMax * 8 + 256);
+    CUDA_CHECK(cudaMemsetAsync(P->dpart.p, 0, P->dpart.bytes, ctx->stream));
     sync(ctx);
 }
 
-// tile: 1 = the quad tile (one 64-thread CTA per block), 2, 4, 8, 16 = the
-// slab tile with that many z-planes per 256-thread CTA.
+// z-planes of a quad-tile CTA: 4 while that leaves the chip less than full
+// (776 blocks: a PCG solve 3.60 ms with 16, 3.50 ms with 4), 16 where whole
+// blocks fill it and splitting only re-reads planes.
+constexpr int64_t kQuadSplitMax = 2048;
+static int quad_planes(int64_t n_blocks) { return n_blocks <= kQuadSplitMax ? 4 : 16; }
+
+template <int OP, bool DOT = false>
+static void launch_quad16(msbg_ctx* ctx, const PLevelDev& L, const float* x, const float* b, float* out, float omega,
+                          const DotArgs& dot = DotArgs{}) {
+    const LevelArgs a = level_args(L);
+    if (quad_planes(L.n()) == 4) pk_quad16<OP, 4, DOT><<<(unsigned)L.n() * 4, 64, 0, ctx->stream>>>(a, x, b, out, omega, dot);
+    else pk_quad16<OP, 16, DOT><<<(unsigned)L.n(), 64, 0, ctx->stream>>>(a, x, b, out, omega, dot);
+}
+
+// tile: 1 = the quad tile (64-thread CTAs), 2, 4, 8, 16 = the slab tile with
+// that many z-planes per 256-thread CTA.
 template <int OP>
 static void launch_block16(msbg_ctx* ctx, const PLevelDev& L, int slab, const float* x, const float* b, float* out,
                            float omega) {
     const LevelArgs a = level_args(L);
     if (slab == 1) {
-        pk_quad16<OP><<<(unsigned)L.n(), 64, 0, ctx->stream>>>(a, x, b, out, omega);
+        launch_quad16<OP>(ctx, L, x, b, out, omega);
         return;
     }
     const unsigned grid = (unsigned)(L.n() * (16 / slab));
@@ -969,6 +1074,8 @@ static void launch_block16(msbg_ctx* ctx, const PLevelDev& L, int slab, const fl
     }
 }
 static bool uses_block16(const PLevelDev& L) { return L.lg == 4 && !L.diag.p; }
+// Whether level 0's kernels can form CG's dot products themselves.
+static bool fuses_dots(const PLevelDev& L) { return uses_block16(L) && L.n() * (16 / quad_planes(L.n())) <= kFusedDotMax; }
 
 static void launch_matvec(msbg_poisson* P, int l, const float* x, float* y) {
     const PLevelDev& L = P->lv[l];
@@ -996,7 +1103,9 @@ static void launch_residual(msbg_poisson* P, int l, const float* x, const float*
 
 // `sweeps` Jacobi sweeps on x (in place through the level's t buffer); x_zero
 // marks x as all zeros on entry.
-static void jacobi(msbg_poisson* P, int l, float* x, const float* b, int sweeps, float omega, bool x_zero) {
+// `dot` (level 0 where fuses_dots): b . x of the result, formed by the last sweep.
+static void jacobi(msbg_poisson* P, int l, float* x, const float* b, int sweeps, float omega, bool x_zero,
+                   const DotArgs* dot = nullptr) {
     PLevelDev& L = P->lv[l];
     float* t = L.t.as<float>();
     int s = 0;
@@ -1017,6 +1126,11 @@ static void jacobi(msbg_poisson* P, int l, float* x, const float* b, int sweeps,
         const float* src = (s % 2 == 0) ? x : t;
         float* dst = (s % 2 == 0) ? t : x;
         begin_launch(P->ctx);
+        if (dot && s == sweeps - 1) {
+            launch_quad16<0, true>(P->ctx, L, src, b, dst, omega, *dot);
+            after_launch(P->ctx, "pk_block16_jacobi");
+            continue;
+        }
         if (uses_block16(L)) {
             launch_block16<0>(P->ctx, L, L.slab, (s == 0 && x_zero) ? nullptr : src, b, dst, omega);
             after_launch(P->ctx, "pk_block16_jacobi");
@@ -1029,8 +1143,9 @@ static void jacobi(msbg_poisson* P, int l, float* x, const float* b, int sweeps,
     if (sweeps % 2 == 1) CUDA_CHECK(cudaMemcpyAsync(x, t, L.cells() * 4, cudaMemcpyDeviceToDevice, P->ctx->stream));
 }
 
-// One V-cycle on level l: x_l improved for A_l x_l = b_l (x_zero: x_l = 0 on entry).
-static void vcycle(msbg_poisson* P, int l, float* x, const float* b, bool x_zero) {
+// One V-cycle on level l: x_l improved for A_l x_l = b_l (x_zero: x_l = 0 on
+// entry).  `dot`: b . x of the result, formed by the last sweep.
+static void vcycle(msbg_poisson* P, int l, float* x, const float* b, bool x_zero, const DotArgs* dot = nullptr) {
     if (l == (int)P->lv.size() - 1) {
         begin_launch(P->ctx);
         pk_dense_solve<<<grid_for(P->nc * 32), 256, 0, P->ctx->stream>>>(P->ainv.as<double>(), P->nc, b, x);
@@ -1069,7 +1184,7 @@ static void vcycle(msbg_poisson* P, int l, float* x, const float* b, bool x_zero
         pk_prolong<<<grid_for(F.cells()), 256, 0, P->ctx->stream>>>(T, C.x.as<float>(), x);
         after_launch(P->ctx, "pk_prolong");
     }
-    jacobi(P, l, x, b, P->nu2, P->omega, false);
+    jacobi(P, l, x, b, P->nu2, P->omega, false, dot);
 }
 
 static double dot(msbg_poisson* P, const float* a, const float* b, int64_t n) {
@@ -1200,13 +1315,29 @@ static int solve_loop(msbg_poisson* P, int method, const float* b, double* x64, 
     double* hist = P->shist.as<double>();
     msbg_poisson::SGraph* g = nullptr;
     for (auto& v : P->sgraphs)
-        if (v.method == method && v.b == b && v.x64 == x64) g = &v;
+        if (v.method == method && v.b == (method == 0 ? b : nullptr) && v.x64 == x64) g = &v;
     if (!g) {
+        const PLevelDev& F = P->lv[0];
+        const bool fused = method == 1 && fuses_dots(F) && P->nu2 >= 1;
+        auto dot_args = [&](int kind) {
+            return DotArgs{P->dpart.as<double>(), (unsigned int*)(P->dpart.as<double>() + kFusedDotMax), sc, kind, {}, ctl, hist};
+        };
         auto cg_step = [&](cudaGraphConditionalHandle h) {  // q = A p, alpha, x += alpha p, r -= alpha q, r.r, test
+            if (fused) {
+                begin_launch(ctx);
+                launch_quad16<2, true>(ctx, F, p, nullptr, q, 0.0f, dot_args(DOT_PQ));
+                after_launch(ctx, "pk_block16_matvec");
+                DotArgs rr = dot_args(DOT_RR);
+                rr.cond = h;
+                begin_launch(ctx);
+                pk_cg_update<true><<<grid_for(n), 256, 0, ctx->stream>>>(n, sc, p, q, x64, r, rr);
+                after_launch(ctx, "pk_cg_update");
+                return;
+            }
             launch_matvec(P, 0, p, q);
             dot_dev(P, p, q, n, SC_PQ);
             begin_launch(ctx);
-            pk_cg_update<<<grid_for(n), 256, 0, ctx->stream>>>(n, sc, p, q, x64, r);
+            pk_cg_update<false><<<grid_for(n), 256, 0, ctx->stream>>>(n, sc, p, q, x64, r, DotArgs{});
             after_launch(ctx, "pk_cg_update");
             dot_dev(P, r, r, n, SC_RR);
             begin_launch(ctx);
@@ -1229,9 +1360,10 @@ static int solve_loop(msbg_poisson* P, int method, const float* b, double* x64, 
             if (method == 1) {
                 CUDA_CHECK(cudaStreamBeginCaptureToGraph(ctx->stream, G, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
                 capturing = true;
-                vcycle(P, 0, z, r, true);
+                const DotArgs rz = dot_args(DOT_RZ);
+                vcycle(P, 0, z, r, true, fused ? &rz : nullptr);
                 CUDA_CHECK(cudaMemcpyAsync(p, z, n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
-                dot_dev(P, r, z, n, SC_RZ);
+                if (!fused) dot_dev(P, r, z, n, SC_RZ);
                 cg_step(h);
                 CUDA_CHECK(cudaStreamEndCapture(ctx->stream, &G));
                 capturing = false;
@@ -1258,7 +1390,8 @@ static int solve_loop(msbg_poisson* P, int method, const float* b, double* x64, 
             const uint64_t l1 = ctx->launches;
             CUDA_CHECK(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
             capturing = true;
-            vcycle(P, 0, z, r, true);
+            const DotArgs rz2 = dot_args(DOT_RZ2);
+            vcycle(P, 0, z, r, true, fused ? &rz2 : nullptr);
             if (method == 0) {
                 add64(P, n, 1.0, z, x64);
                 launch_residual64(P, x64, b, r);
@@ -1267,10 +1400,12 @@ static int solve_loop(msbg_poisson* P, int method, const float* b, double* x64, 
                 pk_solve_test<<<1, 1, 0, ctx->stream>>>(h, sc, ctl, hist, 0);
                 after_launch(ctx, "pk_solve_test");
             } else {
-                dot_dev(P, r, z, n, SC_RZ2);
-                begin_launch(ctx);
-                pk_cg_beta<<<1, 1, 0, ctx->stream>>>(sc, 0);
-                after_launch(ctx, "pk_cg_beta");
+                if (!fused) {
+                    dot_dev(P, r, z, n, SC_RZ2);
+                    begin_launch(ctx);
+                    pk_cg_beta<<<1, 1, 0, ctx->stream>>>(sc, 0);
+                    after_launch(ctx, "pk_cg_beta");
+                }
                 begin_launch(ctx);
                 pk_cg_direction<<<grid_for(n), 256, 0, ctx->stream>>>(n, sc, z, p);
                 after_launch(ctx, "pk_cg_direction");
@@ -1291,7 +1426,7 @@ static int solve_loop(msbg_poisson* P, int method, const float* b, double* x64, 
         }
         cudaGraphDestroy(G);
         ctx->launches = l0;
-        P->sgraphs.push_back({method, b, x64, exec, k_first, k_body});
+        P->sgraphs.push_back({method, method == 0 ? b : nullptr, x64, exec, k_first, k_body});
         g = &P->sgraphs.back();
     }
     const SolveCtl c0{it0, max_iter, thr, bn};
@@ -1491,7 +1626,7 @@ static int solve(msbg_poisson* P, int method, float* x, const float* b, double t
                 dot_dev(P, p, q, n, SC_PQ);
                 if (flexible) CUDA_CHECK(cudaMemcpyAsync(r_old, r, n * 4, cudaMemcpyDeviceToDevice, P->ctx->stream));
                 begin_launch(P->ctx);
-                pk_cg_update<<<grid_for(n), 256, 0, P->ctx->stream>>>(n, sc, p, q, x64, r);
+                pk_cg_update<false><<<grid_for(n), 256, 0, P->ctx->stream>>>(n, sc, p, q, x64, r, DotArgs{});
                 after_launch(P->ctx, "pk_cg_update");
                 dot_dev(P, r, r, n, SC_RR);
                 read_scalars(P, hs);
