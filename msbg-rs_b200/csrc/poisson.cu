@@ -168,7 +168,9 @@ __device__ __forceinline__ T nb_sum(const LevelArgs& L, const T* __restrict__ x,
 }
 
 // y = A x
-__global__ void pk_matvec(LevelArgs L, const float* __restrict__ x, float* __restrict__ y) {
+__global__ void pk_matvec(LevelArgs L, const float* x, float* __restrict__ y) {
+    chain_trigger();
+    chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < L.cells; i += (int64_t)gridDim.x * blockDim.x) {
         if (!L.diag) y[i] = L.scale * (6.0f * x[i] - nb_sum(L, x, i));
         else {
@@ -179,7 +181,9 @@ __global__ void pk_matvec(LevelArgs L, const float* __restrict__ x, float* __res
 }
 
 // r = b - A x (0 at inactive cells)
-__global__ void pk_residual(LevelArgs L, const float* __restrict__ x, const float* __restrict__ b, float* __restrict__ r) {
+__global__ void pk_residual(LevelArgs L, const float* x, const float* b, float* __restrict__ r) {
+    chain_trigger();
+    chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < L.cells; i += (int64_t)gridDim.x * blockDim.x) {
         if (!L.diag) r[i] = b[i] - L.scale * (6.0f * x[i] - nb_sum(L, x, i));
         else {
@@ -193,32 +197,38 @@ __global__ void pk_residual(LevelArgs L, const float* __restrict__ x, const floa
 // f32.  The solution of a solve accumulates in FP64: with an f32 solution the
 // rounding of x alone leaves a relative residual of order 6 eps / lambda_min,
 // about 1e-5 on thin shells, above the 1e-6 target.
-__global__ void pk_residual64(LevelArgs L, const double* __restrict__ x, const float* __restrict__ b,
+__global__ void pk_residual64(LevelArgs L, const double* x, const float* b,
                               float* __restrict__ r) {
+    chain_trigger();
+    chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < L.cells; i += (int64_t)gridDim.x * blockDim.x)
         r[i] = (float)((double)b[i] - (double)L.scale * (6.0 * x[i] - nb_sum(L, x, i)));
 }
 
 // x += a * d (x FP64, d f32)
-__global__ void pk_add64(int64_t n, double a, const float* __restrict__ d, double* __restrict__ x) {
+__global__ void pk_add64(int64_t n, double a, const float* d, double* __restrict__ x) {
+    chain_trigger();
+    chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         x[i] += a * (double)d[i];
 }
 
-__global__ void pk_widen(int64_t n, const float* __restrict__ s, double* __restrict__ d) {
+__global__ void pk_widen(int64_t n, const float* s, double* __restrict__ d) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         d[i] = (double)s[i];
 }
 
-__global__ void pk_narrow(int64_t n, const double* __restrict__ s, float* __restrict__ d) {
+__global__ void pk_narrow(int64_t n, const double* s, float* __restrict__ d) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         d[i] = (float)s[i];
 }
 
 // One weighted Jacobi sweep: xn = w (b + s sum_nb x) / (6 s) + (1 - w) x.
 // x == null means x = 0.
-__global__ void pk_jacobi(LevelArgs L, const float* __restrict__ x, const float* __restrict__ b, float* __restrict__ xn,
+__global__ void pk_jacobi(LevelArgs L, const float* x, const float* b, float* __restrict__ xn,
                           float omega) {
+    chain_trigger();
+    chain_wait();
     const float inv_d = 1.0f / (6.0f * L.scale);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < L.cells; i += (int64_t)gridDim.x * blockDim.x) {
         if (!L.diag) {
@@ -239,7 +249,9 @@ __global__ void pk_jacobi(LevelArgs L, const float* __restrict__ x, const float*
 // formed where the second sweep reads it, with pk_jacobi's operations, so the
 // result is the two sweeps' bits (x1's products rounded on their own, as
 // when x1 is stored, not fused into the neighbour sum).
-__global__ void pk_jacobi_zero2(LevelArgs L, const float* __restrict__ b, float* __restrict__ xn, float omega) {
+__global__ void pk_jacobi_zero2(LevelArgs L, const float* b, float* __restrict__ xn, float omega) {
+    chain_trigger();
+    chain_wait();
     const float inv_d = 1.0f / (6.0f * L.scale);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < L.cells; i += (int64_t)gridDim.x * blockDim.x) {
         if (!L.diag) {
@@ -288,7 +300,7 @@ __device__ __forceinline__ float nb6(float xm, float xp, float ym, float yp, flo
 // above in registers (the next one prefetched), the current plane and its
 // x/y halo from the face neighbours in shared memory.
 template <int OP, int SLAB>
-__global__ void __launch_bounds__(256) pk_block16(LevelArgs L, const float* __restrict__ x, const float* __restrict__ b,
+__global__ void __launch_bounds__(256) pk_block16(LevelArgs L, const float* x, const float* b,
                                                   float* __restrict__ out, float omega) {
     __shared__ float pl[18][18];
     __shared__ int32_t nb[6];
@@ -298,12 +310,14 @@ __global__ void __launch_bounds__(256) pk_block16(LevelArgs L, const float* __re
     const int col = tx + (ty << 4);
     const int64_t base = k << 12;
     const float inv_d = 1.0f / (6.0f * L.scale);
+    chain_trigger();
+    if (threadIdx.x < 6) nb[threadIdx.x] = L.nbr[k * 6 + threadIdx.x];
+    chain_wait();
     if (OP == 0 && !x) {
         for (int z = z0; z < z0 + SLAB; ++z)
             out[base + col + (z << 8)] = __fmul_rn(__fmul_rn(omega, b[base + col + (z << 8)]), inv_d);
         return;
     }
-    if (threadIdx.x < 6) nb[threadIdx.x] = L.nbr[k * 6 + threadIdx.x];
     __syncthreads();
     const int32_t nxm = nb[0], nxp = nb[1], nym = nb[2], nyp = nb[3], nzm = nb[4], nzp = nb[5];
     // the value the sweep reads at x[j]: x1 = w b inv_d for OP 3
@@ -450,7 +464,7 @@ __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast
 __device__ __forceinline__ float comp(const float4& v, int e) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; }
 
 template <int OP, int ZS, bool DOT = false>
-__global__ void __launch_bounds__(64) pk_quad16(LevelArgs L, const float* __restrict__ x, const float* __restrict__ b,
+__global__ void __launch_bounds__(64) pk_quad16(LevelArgs L, const float* x, const float* b,
                                                 float* __restrict__ out, float omega, DotArgs dot) {
     __shared__ float4 pl[2][18][4];  // rows y = -1..16 of a plane, four quads each
     const int64_t k = blockIdx.x / (16 / ZS);
@@ -460,6 +474,11 @@ __global__ void __launch_bounds__(64) pk_quad16(LevelArgs L, const float* __rest
     const int64_t base = k << 12;
     const int off = (y << 4) + (q << 2);
     const float inv_d = 1.0f / (6.0f * L.scale);
+    const int32_t* nbr = L.nbr + k * 6;
+    chain_trigger();
+    const int32_t nxm = __ldg(nbr), nxp = __ldg(nbr + 1), nym = __ldg(nbr + 2), nyp = __ldg(nbr + 3), nzm = __ldg(nbr + 4),
+                  nzp = __ldg(nbr + 5);
+    chain_wait();
     if (OP == 0 && !x) {
         for (int z = z0; z < z0 + ZS; ++z) {
             const float4 bv = ld4(b + base + off + (z << 8));
@@ -469,9 +488,6 @@ __global__ void __launch_bounds__(64) pk_quad16(LevelArgs L, const float* __rest
         }
         return;
     }
-    const int32_t* nbr = L.nbr + k * 6;
-    const int32_t nxm = __ldg(nbr), nxp = __ldg(nbr + 1), nym = __ldg(nbr + 2), nyp = __ldg(nbr + 3), nzm = __ldg(nbr + 4),
-                  nzp = __ldg(nbr + 5);
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     // the values the sweep reads: x1 = w b inv_d for OP 3
     auto tr = [&](float v) -> float { return OP == 3 ? __fmul_rn(__fmul_rn(omega, v), inv_d) : v; };
@@ -531,7 +547,9 @@ struct TransferArgs {
     int64_t cells;          // cells of the level the kernel runs over
 };
 
-__global__ void pk_restrict(TransferArgs T, const float* __restrict__ r, float* __restrict__ bc) {
+__global__ void pk_restrict(TransferArgs T, const float* r, float* __restrict__ bc) {
+    chain_trigger();
+    chain_wait();
     const int bsc = 1 << T.lgc, mc = bsc - 1, mf = (1 << T.lgf) - 1;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T.cells; i += (int64_t)gridDim.x * blockDim.x) {
         if (T.diag && !(T.diag[i] > 0.0f)) {
@@ -572,7 +590,9 @@ __global__ void pk_restrict(TransferArgs T, const float* __restrict__ r, float* 
 }
 
 // x_f += P x_c at the active fine cells.
-__global__ void pk_prolong(TransferArgs T, const float* __restrict__ xc, float* __restrict__ xf) {
+__global__ void pk_prolong(TransferArgs T, const float* xc, float* __restrict__ xf) {
+    chain_trigger();
+    chain_wait();
     const int bsf = 1 << T.lgf, mf = bsf - 1, mc = (1 << T.lgc) - 1;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T.cells; i += (int64_t)gridDim.x * blockDim.x) {
         if (T.diag && !(T.diag[i] > 0.0f)) continue;
@@ -612,17 +632,19 @@ __global__ void pk_prolong(TransferArgs T, const float* __restrict__ xc, float* 
 // NT threads a CTA; the staging loops are unrolled so that a thread's loads
 // are in flight together.
 template <int LGF, int NT>
-__global__ void __launch_bounds__(NT) pk_restrict_tile(TransferArgs T, const float* __restrict__ r, float* __restrict__ bc) {
+__global__ void __launch_bounds__(NT) pk_restrict_tile(TransferArgs T, const float* r, float* __restrict__ bc) {
     constexpr int BF = 1 << LGF, BC = BF / 2, LGC = LGF - 1, W = BF + 2, NC = BC * BC * BC;
     __shared__ float f[W * W * W];  // fine cells -1 .. BF of the fine block under coarse block k
     __shared__ int32_t fs[27];
     const int64_t k = blockIdx.x;
+    chain_trigger();
     if (threadIdx.x < 27) {
         // fine block at offset (t % 3, t / 3 % 3, t / 9) - 1; the restriction table starts at offset -1
         const int t = threadIdx.x;
         fs[t] = T.nb[k * 64 + (t % 3) + 4 * ((t / 3) % 3) + 16 * (t / 9)];
     }
     __syncthreads();
+    chain_wait();
 #pragma unroll
     for (int e0 = 0; e0 < W * W * W; e0 += NT) {
         const int e = e0 + (int)threadIdx.x;
@@ -659,13 +681,15 @@ __global__ void __launch_bounds__(NT) pk_restrict_tile(TransferArgs T, const flo
 }
 
 template <int LGF, int NT>
-__global__ void __launch_bounds__(NT) pk_prolong_tile(TransferArgs T, const float* __restrict__ xc, float* __restrict__ xf) {
+__global__ void __launch_bounds__(NT) pk_prolong_tile(TransferArgs T, const float* xc, float* __restrict__ xf) {
     constexpr int BF = 1 << LGF, BC = BF / 2, LGC = LGF - 1, W = BC + 2, NF = BF * BF * BF;
     __shared__ float c[W * W * W];  // coarse cells -1 .. BC of fine block k's parent
     __shared__ int32_t cs[27];
     const int64_t k = blockIdx.x;
+    chain_trigger();
     if (threadIdx.x < 27) cs[threadIdx.x] = T.nb[k * 27 + threadIdx.x];
     __syncthreads();
+    chain_wait();
 #pragma unroll
     for (int e0 = 0; e0 < W * W * W; e0 += NT) {
         const int e = e0 + (int)threadIdx.x;
@@ -703,7 +727,9 @@ __global__ void __launch_bounds__(NT) pk_prolong_tile(TransferArgs T, const floa
 // the symmetric operator is symmetric, so row i is column i: its n entries
 // are contiguous and the warp reads them coalesced.  Lane partial sums are
 // combined in a fixed butterfly order (deterministic).
-__global__ void pk_dense_solve(const double* __restrict__ ainv, int64_t n, const float* __restrict__ b, float* __restrict__ x) {
+__global__ void pk_dense_solve(const double* ainv, int64_t n, const float* b, float* __restrict__ x) {
+    chain_trigger();
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
@@ -720,8 +746,10 @@ __global__ void pk_dense_solve(const double* __restrict__ ainv, int64_t n, const
 constexpr int DOT_THREADS = 256;
 constexpr int DOT_BLOCKS = 1184;  // 8 per SM
 
-__global__ void __launch_bounds__(DOT_THREADS) pk_dot_partial(const float* __restrict__ a, const float* __restrict__ b,
+__global__ void __launch_bounds__(DOT_THREADS) pk_dot_partial(const float* a, const float* b,
                                                                int64_t n, double* __restrict__ partial) {
+    chain_trigger();
+    chain_wait();
     __shared__ double sm[DOT_THREADS];
     double s = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)DOT_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * DOT_THREADS)
@@ -735,7 +763,9 @@ __global__ void __launch_bounds__(DOT_THREADS) pk_dot_partial(const float* __res
     if (threadIdx.x == 0) partial[blockIdx.x] = sm[0];
 }
 
-__global__ void __launch_bounds__(DOT_THREADS) pk_dot_final(const double* __restrict__ partial, int np, double* __restrict__ out) {
+__global__ void __launch_bounds__(DOT_THREADS) pk_dot_final(const double* partial, int np, double* __restrict__ out) {
+    chain_trigger();
+    chain_wait();
     __shared__ double sm[DOT_THREADS];
     double s = 0.0;
     for (int i = threadIdx.x; i < np; i += DOT_THREADS) s += partial[i];
@@ -749,14 +779,16 @@ __global__ void __launch_bounds__(DOT_THREADS) pk_dot_final(const double* __rest
 }
 
 // y = a*x + b*y (f32 vectors, scalars from FP64)
-__global__ void pk_axpby(int64_t n, float a, const float* __restrict__ x, float b, float* __restrict__ y) {
+__global__ void pk_axpby(int64_t n, float a, const float* x, float b, float* __restrict__ y) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] = a * x[i] + b * y[i];
 }
 
 // Stage 2 of p.Ap (the same tree as pk_dot_final), then alpha = r.z / p.Ap.
-__global__ void __launch_bounds__(DOT_THREADS) pk_dot_final_alpha(const double* __restrict__ partial, int np,
+__global__ void __launch_bounds__(DOT_THREADS) pk_dot_final_alpha(const double* partial, int np,
                                                                    double* __restrict__ sc) {
+    chain_trigger();
+    chain_wait();
     __shared__ double sm[DOT_THREADS];
     double s = 0.0;
     for (int i = threadIdx.x; i < np; i += DOT_THREADS) s += partial[i];
@@ -772,9 +804,11 @@ __global__ void __launch_bounds__(DOT_THREADS) pk_dot_final_alpha(const double* 
 // x += alpha p (FP64) and r = (-alpha) q + r (f32) as fused multiply-adds,
 // skipped on breakdown.  DOT: r.r of the new residual and the loop's test.
 template <bool DOT>
-__global__ void __launch_bounds__(256) pk_cg_update(int64_t n, const double* __restrict__ sc, const float* __restrict__ p,
-                                                    const float* __restrict__ q, double* __restrict__ x, float* __restrict__ r,
+__global__ void __launch_bounds__(256) pk_cg_update(int64_t n, const double* sc, const float* p,
+                                                    const float* q, double* __restrict__ x, float* __restrict__ r,
                                                     DotArgs dot) {
+    chain_trigger();
+    chain_wait();
     const bool bad = sc[SC_BAD] != 0.0;
     if (!DOT && bad) return;
     const double a = sc[SC_ALPHA];
@@ -792,11 +826,17 @@ __global__ void __launch_bounds__(256) pk_cg_update(int64_t n, const double* __r
     if (DOT) dot_finish<256>(s, dot);
 }
 
-__global__ void pk_cg_beta(double* __restrict__ sc, int flexible) { cg_beta(sc, flexible); }
+__global__ void pk_cg_beta(double* __restrict__ sc, int flexible) {
+    chain_trigger();
+    chain_wait();
+    cg_beta(sc, flexible);
+}
 
 // p = z + beta p (f32; beta from the device; the product rounded, then the sum)
-__global__ void pk_cg_direction(int64_t n, const double* __restrict__ sc, const float* __restrict__ z,
+__global__ void pk_cg_direction(int64_t n, const double* sc, const float* z,
                                 float* __restrict__ p) {
+    chain_trigger();
+    chain_wait();
     const float b = (float)sc[SC_BETA];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         p[i] = __fadd_rn(z[i], __fmul_rn(b, p[i]));
@@ -822,8 +862,10 @@ static LevelArgs level_args(const PLevelDev& L) {
     return LevelArgs{L.nbr.as<int32_t>(), L.lg, L.cells(), L.scale, L.diag.p ? L.diag.as<float>() : nullptr};
 }
 
-__global__ void pk_solve_test(cudaGraphConditionalHandle h, const double* __restrict__ sc, SolveCtl* __restrict__ c,
+__global__ void pk_solve_test(cudaGraphConditionalHandle h, const double* sc, SolveCtl* __restrict__ c,
                               double* __restrict__ hist, int check_bad) {
+    chain_trigger();
+    chain_wait();
     solve_test(h, sc, c, hist, check_bad);
 }
 
@@ -1051,8 +1093,8 @@ template <int OP, bool DOT = false>
 static void launch_quad16(msbg_ctx* ctx, const PLevelDev& L, const float* x, const float* b, float* out, float omega,
                           const DotArgs& dot = DotArgs{}) {
     const LevelArgs a = level_args(L);
-    if (quad_planes(L.n()) == 4) pk_quad16<OP, 4, DOT><<<(unsigned)L.n() * 4, 64, 0, ctx->stream>>>(a, x, b, out, omega, dot);
-    else pk_quad16<OP, 16, DOT><<<(unsigned)L.n(), 64, 0, ctx->stream>>>(a, x, b, out, omega, dot);
+    if (quad_planes(L.n()) == 4) launch_chained(ctx->stream, pk_quad16<OP, 4, DOT>, (unsigned)L.n() * 4, 64, 0, 1, a, x, b, out, omega, dot);
+    else launch_chained(ctx->stream, pk_quad16<OP, 16, DOT>, (unsigned)L.n(), 64, 0, 1, a, x, b, out, omega, dot);
 }
 
 // tile: 1 = the quad tile (64-thread CTAs), 2, 4, 8, 16 = the slab tile with
@@ -1067,10 +1109,10 @@ static void launch_block16(msbg_ctx* ctx, const PLevelDev& L, int slab, const fl
     }
     const unsigned grid = (unsigned)(L.n() * (16 / slab));
     switch (slab) {
-        case 2: pk_block16<OP, 2><<<grid, 256, 0, ctx->stream>>>(a, x, b, out, omega); break;
-        case 8: pk_block16<OP, 8><<<grid, 256, 0, ctx->stream>>>(a, x, b, out, omega); break;
-        case 16: pk_block16<OP, 16><<<grid, 256, 0, ctx->stream>>>(a, x, b, out, omega); break;
-        default: pk_block16<OP, 4><<<(unsigned)(L.n() * 4), 256, 0, ctx->stream>>>(a, x, b, out, omega); break;
+        case 2: launch_chained(ctx->stream, pk_block16<OP, 2>, grid, 256, 0, 1, a, x, b, out, omega); break;
+        case 8: launch_chained(ctx->stream, pk_block16<OP, 8>, grid, 256, 0, 1, a, x, b, out, omega); break;
+        case 16: launch_chained(ctx->stream, pk_block16<OP, 16>, grid, 256, 0, 1, a, x, b, out, omega); break;
+        default: launch_chained(ctx->stream, pk_block16<OP, 4>, (unsigned)(L.n() * 4), 256, 0, 1, a, x, b, out, omega); break;
     }
 }
 static bool uses_block16(const PLevelDev& L) { return L.lg == 4 && !L.diag.p; }
@@ -1085,7 +1127,7 @@ static void launch_matvec(msbg_poisson* P, int l, const float* x, float* y) {
         after_launch(P->ctx, "pk_block16_matvec");
         return;
     }
-    pk_matvec<<<grid_for(L.cells()), 256, 0, P->ctx->stream>>>(level_args(L), x, y);
+    launch_chained(P->ctx->stream, pk_matvec, grid_for(L.cells()), 256, 0, 1, level_args(L), x, y);
     after_launch(P->ctx, "pk_matvec");
 }
 
@@ -1097,7 +1139,7 @@ static void launch_residual(msbg_poisson* P, int l, const float* x, const float*
         after_launch(P->ctx, "pk_block16_residual");
         return;
     }
-    pk_residual<<<shape_grid(L.cfg_res, L.cells()), kShapes[L.cfg_res].threads, 0, P->ctx->stream>>>(level_args(L), x, b, r);
+    launch_chained(P->ctx->stream, pk_residual, shape_grid(L.cfg_res, L.cells()), kShapes[L.cfg_res].threads, 0, 1, level_args(L), x, b, r);
     after_launch(P->ctx, "pk_residual");
 }
 
@@ -1116,8 +1158,7 @@ static void jacobi(msbg_poisson* P, int l, float* x, const float* b, int sweeps,
             launch_block16<3>(P->ctx, L, L.slab, b, b, x, omega);
             after_launch(P->ctx, "pk_block16_jacobi0");
         } else {
-            pk_jacobi_zero2<<<shape_grid(L.cfg_jac, L.cells()), kShapes[L.cfg_jac].threads, 0, P->ctx->stream>>>(
-                level_args(L), b, x, omega);
+            launch_chained(P->ctx->stream, pk_jacobi_zero2, shape_grid(L.cfg_jac, L.cells()), kShapes[L.cfg_jac].threads, 0, 1, level_args(L), b, x, omega);
             after_launch(P->ctx, "pk_jacobi_zero2");
         }
         s = 2;
@@ -1136,8 +1177,7 @@ static void jacobi(msbg_poisson* P, int l, float* x, const float* b, int sweeps,
             after_launch(P->ctx, "pk_block16_jacobi");
             continue;
         }
-        pk_jacobi<<<shape_grid(L.cfg_jac, L.cells()), kShapes[L.cfg_jac].threads, 0, P->ctx->stream>>>(
-            level_args(L), (s == 0 && x_zero) ? nullptr : src, b, dst, omega);
+        launch_chained(P->ctx->stream, pk_jacobi, shape_grid(L.cfg_jac, L.cells()), kShapes[L.cfg_jac].threads, 0, 1, level_args(L), (s == 0 && x_zero) ? nullptr : src, b, dst, omega);
         after_launch(P->ctx, "pk_jacobi");
     }
     if (sweeps % 2 == 1) CUDA_CHECK(cudaMemcpyAsync(x, t, L.cells() * 4, cudaMemcpyDeviceToDevice, P->ctx->stream));
@@ -1148,7 +1188,7 @@ static void jacobi(msbg_poisson* P, int l, float* x, const float* b, int sweeps,
 static void vcycle(msbg_poisson* P, int l, float* x, const float* b, bool x_zero, const DotArgs* dot = nullptr) {
     if (l == (int)P->lv.size() - 1) {
         begin_launch(P->ctx);
-        pk_dense_solve<<<grid_for(P->nc * 32), 256, 0, P->ctx->stream>>>(P->ainv.as<double>(), P->nc, b, x);
+        launch_chained(P->ctx->stream, pk_dense_solve, grid_for(P->nc * 32), 256, 0, 1, P->ainv.as<double>(), P->nc, b, x);
         after_launch(P->ctx, "pk_dense_solve");
         return;
     }
@@ -1162,12 +1202,12 @@ static void vcycle(msbg_poisson* P, int l, float* x, const float* b, bool x_zero
     begin_launch(P->ctx);
     if (same_grid) {
         const unsigned nb = (unsigned)C.n();
-        if (F.lg == 4) pk_restrict_tile<4, 256><<<nb, 256, 0, P->ctx->stream>>>(R, F.r.as<float>(), C.b.as<float>());
-        else if (F.lg == 3) pk_restrict_tile<3, 128><<<nb, 128, 0, P->ctx->stream>>>(R, F.r.as<float>(), C.b.as<float>());
-        else pk_restrict_tile<2, 64><<<nb, 64, 0, P->ctx->stream>>>(R, F.r.as<float>(), C.b.as<float>());
+        if (F.lg == 4) launch_chained(P->ctx->stream, pk_restrict_tile<4, 256>, nb, 256, 0, 1, R, F.r.as<float>(), C.b.as<float>());
+        else if (F.lg == 3) launch_chained(P->ctx->stream, pk_restrict_tile<3, 128>, nb, 128, 0, 1, R, F.r.as<float>(), C.b.as<float>());
+        else launch_chained(P->ctx->stream, pk_restrict_tile<2, 64>, nb, 64, 0, 1, R, F.r.as<float>(), C.b.as<float>());
         after_launch(P->ctx, "pk_restrict_tile");
     } else {
-        pk_restrict<<<grid_for(C.cells()), 256, 0, P->ctx->stream>>>(R, F.r.as<float>(), C.b.as<float>());
+        launch_chained(P->ctx->stream, pk_restrict, grid_for(C.cells()), 256, 0, 1, R, F.r.as<float>(), C.b.as<float>());
         after_launch(P->ctx, "pk_restrict");
     }
     vcycle(P, l + 1, C.x.as<float>(), C.b.as<float>(), true);
@@ -1176,12 +1216,12 @@ static void vcycle(msbg_poisson* P, int l, float* x, const float* b, bool x_zero
     begin_launch(P->ctx);
     if (same_grid) {
         const unsigned nb = (unsigned)F.n();
-        if (F.lg == 4) pk_prolong_tile<4, 256><<<nb, 256, 0, P->ctx->stream>>>(T, C.x.as<float>(), x);
-        else if (F.lg == 3) pk_prolong_tile<3, 256><<<nb, 256, 0, P->ctx->stream>>>(T, C.x.as<float>(), x);
-        else pk_prolong_tile<2, 64><<<nb, 64, 0, P->ctx->stream>>>(T, C.x.as<float>(), x);
+        if (F.lg == 4) launch_chained(P->ctx->stream, pk_prolong_tile<4, 256>, nb, 256, 0, 1, T, C.x.as<float>(), x);
+        else if (F.lg == 3) launch_chained(P->ctx->stream, pk_prolong_tile<3, 256>, nb, 256, 0, 1, T, C.x.as<float>(), x);
+        else launch_chained(P->ctx->stream, pk_prolong_tile<2, 64>, nb, 64, 0, 1, T, C.x.as<float>(), x);
         after_launch(P->ctx, "pk_prolong_tile");
     } else {
-        pk_prolong<<<grid_for(F.cells()), 256, 0, P->ctx->stream>>>(T, C.x.as<float>(), x);
+        launch_chained(P->ctx->stream, pk_prolong, grid_for(F.cells()), 256, 0, 1, T, C.x.as<float>(), x);
         after_launch(P->ctx, "pk_prolong");
     }
     jacobi(P, l, x, b, P->nu2, P->omega, false, dot);
@@ -1190,10 +1230,10 @@ static void vcycle(msbg_poisson* P, int l, float* x, const float* b, bool x_zero
 static double dot(msbg_poisson* P, const float* a, const float* b, int64_t n) {
     double* part = (double*)((char*)P->work.p + P->work.bytes - (DOT_BLOCKS + 16) * 8);
     begin_launch(P->ctx);
-    pk_dot_partial<<<DOT_BLOCKS, DOT_THREADS, 0, P->ctx->stream>>>(a, b, n, part);
+    launch_chained(P->ctx->stream, pk_dot_partial, DOT_BLOCKS, DOT_THREADS, 0, 1, a, b, n, part);
     after_launch(P->ctx, "pk_dot_partial");
     begin_launch(P->ctx);
-    pk_dot_final<<<1, DOT_THREADS, 0, P->ctx->stream>>>(part, DOT_BLOCKS, part + DOT_BLOCKS);
+    launch_chained(P->ctx->stream, pk_dot_final, 1, DOT_THREADS, 0, 1, part, DOT_BLOCKS, part + DOT_BLOCKS);
     after_launch(P->ctx, "pk_dot_final");
     double h = 0.0;
     read_small(P->ctx, &h, part + DOT_BLOCKS, 8);
@@ -1210,14 +1250,14 @@ static void dot_dev(msbg_poisson* P, const float* a, const float* b, int64_t n, 
     double* part = (double*)((char*)P->work.p + P->work.bytes - (DOT_BLOCKS + 16) * 8);
     double* sc = cg_scalars(P);
     begin_launch(P->ctx);
-    pk_dot_partial<<<DOT_BLOCKS, DOT_THREADS, 0, P->ctx->stream>>>(a, b, n, part);
+    launch_chained(P->ctx->stream, pk_dot_partial, DOT_BLOCKS, DOT_THREADS, 0, 1, a, b, n, part);
     after_launch(P->ctx, "pk_dot_partial");
     begin_launch(P->ctx);
     if (slot == SC_PQ) {
-        pk_dot_final_alpha<<<1, DOT_THREADS, 0, P->ctx->stream>>>(part, DOT_BLOCKS, sc);
+        launch_chained(P->ctx->stream, pk_dot_final_alpha, 1, DOT_THREADS, 0, 1, part, DOT_BLOCKS, sc);
         after_launch(P->ctx, "pk_dot_final_alpha");
     } else {
-        pk_dot_final<<<1, DOT_THREADS, 0, P->ctx->stream>>>(part, DOT_BLOCKS, sc + slot);
+        launch_chained(P->ctx->stream, pk_dot_final, 1, DOT_THREADS, 0, 1, part, DOT_BLOCKS, sc + slot);
         after_launch(P->ctx, "pk_dot_final");
     }
 }
@@ -1234,13 +1274,13 @@ static void axpby(msbg_poisson* P, int64_t n, double a, const float* x, double b
 static void launch_residual64(msbg_poisson* P, const double* x, const float* b, float* r) {
     const PLevelDev& L = P->lv[0];
     begin_launch(P->ctx);
-    pk_residual64<<<grid_for(L.cells()), 256, 0, P->ctx->stream>>>(level_args(L), x, b, r);
+    launch_chained(P->ctx->stream, pk_residual64, grid_for(L.cells()), 256, 0, 1, level_args(L), x, b, r);
     after_launch(P->ctx, "pk_residual64");
 }
 
 static void add64(msbg_poisson* P, int64_t n, double a, const float* d, double* x) {
     begin_launch(P->ctx);
-    pk_add64<<<grid_for(n), 256, 0, P->ctx->stream>>>(n, a, d, x);
+    launch_chained(P->ctx->stream, pk_add64, grid_for(n), 256, 0, 1, n, a, d, x);
     after_launch(P->ctx, "pk_add64");
 }
 
@@ -1330,18 +1370,18 @@ static int solve_loop(msbg_poisson* P, int method, const float* b, double* x64, 
                 DotArgs rr = dot_args(DOT_RR);
                 rr.cond = h;
                 begin_launch(ctx);
-                pk_cg_update<true><<<grid_for(n), 256, 0, ctx->stream>>>(n, sc, p, q, x64, r, rr);
+                launch_chained(ctx->stream, pk_cg_update<true>, grid_for(n), 256, 0, 1, n, sc, p, q, x64, r, rr);
                 after_launch(ctx, "pk_cg_update");
                 return;
             }
             launch_matvec(P, 0, p, q);
             dot_dev(P, p, q, n, SC_PQ);
             begin_launch(ctx);
-            pk_cg_update<false><<<grid_for(n), 256, 0, ctx->stream>>>(n, sc, p, q, x64, r, DotArgs{});
+            launch_chained(ctx->stream, pk_cg_update<false>, grid_for(n), 256, 0, 1, n, sc, p, q, x64, r, DotArgs{});
             after_launch(ctx, "pk_cg_update");
             dot_dev(P, r, r, n, SC_RR);
             begin_launch(ctx);
-            pk_solve_test<<<1, 1, 0, ctx->stream>>>(h, sc, ctl, hist, 1);
+            launch_chained(ctx->stream, pk_solve_test, 1, 1, 0, 1, h, sc, ctl, hist, 1);
             after_launch(ctx, "pk_solve_test");
         };
         cudaGraph_t G = nullptr;
@@ -1397,17 +1437,17 @@ static int solve_loop(msbg_poisson* P, int method, const float* b, double* x64, 
                 launch_residual64(P, x64, b, r);
                 dot_dev(P, r, r, n, SC_RR);
                 begin_launch(ctx);
-                pk_solve_test<<<1, 1, 0, ctx->stream>>>(h, sc, ctl, hist, 0);
+                launch_chained(ctx->stream, pk_solve_test, 1, 1, 0, 1, h, sc, ctl, hist, 0);
                 after_launch(ctx, "pk_solve_test");
             } else {
                 if (!fused) {
                     dot_dev(P, r, z, n, SC_RZ2);
                     begin_launch(ctx);
-                    pk_cg_beta<<<1, 1, 0, ctx->stream>>>(sc, 0);
+                    launch_chained(ctx->stream, pk_cg_beta, 1, 1, 0, 1, sc, 0);
                     after_launch(ctx, "pk_cg_beta");
                 }
                 begin_launch(ctx);
-                pk_cg_direction<<<grid_for(n), 256, 0, ctx->stream>>>(n, sc, z, p);
+                launch_chained(ctx->stream, pk_cg_direction, grid_for(n), 256, 0, 1, n, sc, z, p);
                 after_launch(ctx, "pk_cg_direction");
                 cg_step(h);
             }
@@ -1626,7 +1666,7 @@ static int solve(msbg_poisson* P, int method, float* x, const float* b, double t
                 dot_dev(P, p, q, n, SC_PQ);
                 if (flexible) CUDA_CHECK(cudaMemcpyAsync(r_old, r, n * 4, cudaMemcpyDeviceToDevice, P->ctx->stream));
                 begin_launch(P->ctx);
-                pk_cg_update<false><<<grid_for(n), 256, 0, P->ctx->stream>>>(n, sc, p, q, x64, r, DotArgs{});
+                launch_chained(P->ctx->stream, pk_cg_update<false>, grid_for(n), 256, 0, 1, n, sc, p, q, x64, r, DotArgs{});
                 after_launch(P->ctx, "pk_cg_update");
                 dot_dev(P, r, r, n, SC_RR);
                 read_scalars(P, hs);
@@ -1674,7 +1714,7 @@ static int solve(msbg_poisson* P, int method, float* x, const float* b, double t
                 dot_dev(P, r, z, n, SC_RZ2);
                 if (flexible) dot_dev(P, z, r_old, n, SC_ZR);
                 begin_launch(P->ctx);
-                pk_cg_beta<<<1, 1, 0, P->ctx->stream>>>(sc, flexible ? 1 : 0);
+                launch_chained(P->ctx->stream, pk_cg_beta, 1, 1, 0, 1, sc, flexible ? 1 : 0);
                 after_launch(P->ctx, "pk_cg_beta");
                 if (flexible && pc != PC_MG) {
                     read_scalars(P, hs);
@@ -1684,7 +1724,7 @@ static int solve(msbg_poisson* P, int method, float* x, const float* b, double t
                     }
                 }
                 begin_launch(P->ctx);
-                pk_cg_direction<<<grid_for(n), 256, 0, P->ctx->stream>>>(n, sc, z, p);
+                launch_chained(P->ctx->stream, pk_cg_direction, grid_for(n), 256, 0, 1, n, sc, z, p);
                 after_launch(P->ctx, "pk_cg_direction");
             }
         }
@@ -1703,7 +1743,7 @@ static int solve(msbg_poisson* P, int method, float* x, const float* b, double t
 // divergence of u = sum_i a_i exp(-|x - c_i|^2 / (2 s_i^2)), evaluated at
 // level-0 cell centres: b = sum_i -(a_i . (x - c_i)) / s_i^2 g_i(x).
 // blobs: [n_blobs][7] = (cx, cy, cz, s, ax, ay, az).
-__global__ void pk_blob_rhs(LevelArgs L, const int32_t* __restrict__ coords, const float* __restrict__ blobs, int n_blobs,
+__global__ void pk_blob_rhs(LevelArgs L, const int32_t* __restrict__ coords, const float* blobs, int n_blobs,
                             float* __restrict__ bout) {
     const int bs = 1 << L.lg, m = bs - 1;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < L.cells; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1723,7 +1763,7 @@ __global__ void pk_blob_rhs(LevelArgs L, const int32_t* __restrict__ coords, con
 }
 
 // e = xs - x (FP64 in, f32 out)
-__global__ void pk_sub64(int64_t n, const double* __restrict__ xs, const double* __restrict__ x, float* __restrict__ e) {
+__global__ void pk_sub64(int64_t n, const double* xs, const double* x, float* __restrict__ e) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         e[i] = (float)(xs[i] - x[i]);
 }
@@ -1930,8 +1970,10 @@ static void evaluate(msbg_poisson* P, int n_rhs, int mg_iters, uint64_t seed, do
 enum { S_RZ = 0, S_PQ, S_RZN, S_RR, S_BB, S_ALPHA, S_BETA, S_ACTIVE, S_ITER, S_WIDTH = 16 };
 
 // per-block FP64 partial of a . b (one CTA per block, fixed tree order)
-__global__ void __launch_bounds__(256) bk_block_dot(int64_t nblocks, int cells, const float* __restrict__ a,
-                                                    const float* __restrict__ b, double* __restrict__ part) {
+__global__ void __launch_bounds__(256) bk_block_dot(int64_t nblocks, int cells, const float* a,
+                                                    const float* b, double* __restrict__ part) {
+    chain_trigger();
+    chain_wait();
     __shared__ double sm[256];
     for (int64_t k = blockIdx.x; k < nblocks; k += gridDim.x) {
         double s = 0.0;
@@ -1948,8 +1990,10 @@ __global__ void __launch_bounds__(256) bk_block_dot(int64_t nblocks, int cells, 
 }
 
 // scal[p][slot] = sum of the partials of problem p's blocks (one warp per problem)
-__global__ void bk_seg_sum(int np, const int64_t* __restrict__ pb, const double* __restrict__ part, double* __restrict__ scal,
+__global__ void bk_seg_sum(int np, const int64_t* __restrict__ pb, const double* part, double* __restrict__ scal,
                            int slot) {
+    chain_trigger();
+    chain_wait();
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < np; p += warps) {
@@ -1965,6 +2009,8 @@ __global__ void bk_seg_sum(int np, const int64_t* __restrict__ pb, const double*
 // iteration counted; op 2: active = (r.r > tol^2 b.b).  Problems that are not
 // active get alpha = beta = 0 and stay where they are.
 __global__ void bk_scalars(int np, double* __restrict__ scal, int op, double tol2) {
+    chain_trigger();
+    chain_wait();
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
         double* S = scal + (int64_t)p * S_WIDTH;
         const bool on = S[S_ACTIVE] > 0.0;
@@ -1981,22 +2027,28 @@ __global__ void bk_scalars(int np, double* __restrict__ scal, int op, double tol
 }
 
 // y += sign * s_p x  (s_p = scal[problem of the cell's block][slot])
-__global__ void bk_axpy(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* __restrict__ scal, int slot,
-                        float sign, const float* __restrict__ x, float* __restrict__ y) {
+__global__ void bk_axpy(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* scal, int slot,
+                        float sign, const float* x, float* __restrict__ y) {
+    chain_trigger();
+    chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] += (float)(sign * scal[(int64_t)blk_prob[i >> lg3] * S_WIDTH + slot]) * x[i];
 }
 
 // p = z + beta_p p
-__global__ void bk_xpay(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* __restrict__ scal,
-                        const float* __restrict__ z, float* __restrict__ p) {
+__global__ void bk_xpay(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* scal,
+                        const float* z, float* __restrict__ p) {
+    chain_trigger();
+    chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         p[i] = z[i] + (float)scal[(int64_t)blk_prob[i >> lg3] * S_WIDTH + S_BETA] * p[i];
 }
 
 // x64 += alpha_p p
-__global__ void bk_add64(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* __restrict__ scal,
-                         const float* __restrict__ p, double* __restrict__ x) {
+__global__ void bk_add64(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* scal,
+                         const float* p, double* __restrict__ x) {
+    chain_trigger();
+    chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         x[i] += scal[(int64_t)blk_prob[i >> lg3] * S_WIDTH + S_ALPHA] * (double)p[i];
 }
@@ -2005,18 +2057,17 @@ static void seg_dot(msbg_poisson* P, const float* a, const float* b, int slot) {
     const PLevelDev& F = P->lv[0];
     const int cells = F.bs * F.bs * F.bs;
     begin_launch(P->ctx);
-    bk_block_dot<<<(unsigned)std::min<int64_t>(F.n(), 148 * 8), 256, 0, P->ctx->stream>>>(F.n(), cells, a, b,
+    launch_chained(P->ctx->stream, bk_block_dot, (unsigned)std::min<int64_t>(F.n(), 148 * 8), 256, 0, 1, F.n(), cells, a, b,
                                                                                          P->bpart.as<double>());
     after_launch(P->ctx, "bk_block_dot");
     begin_launch(P->ctx);
-    bk_seg_sum<<<(unsigned)((P->np * 32 + 255) / 256), 256, 0, P->ctx->stream>>>(
-        P->np, P->d_prob_blocks.as<int64_t>(), P->bpart.as<double>(), P->scal.as<double>(), slot);
+    launch_chained(P->ctx->stream, bk_seg_sum, (unsigned)((P->np * 32 + 255) / 256), 256, 0, 1, P->np, P->d_prob_blocks.as<int64_t>(), P->bpart.as<double>(), P->scal.as<double>(), slot);
     after_launch(P->ctx, "bk_seg_sum");
 }
 
 static void scalars(msbg_poisson* P, int op, double tol) {
     begin_launch(P->ctx);
-    bk_scalars<<<(unsigned)((P->np + 127) / 128), 128, 0, P->ctx->stream>>>(P->np, P->scal.as<double>(), op, tol * tol);
+    launch_chained(P->ctx->stream, bk_scalars, (unsigned)((P->np + 127) / 128), 128, 0, 1, P->np, P->scal.as<double>(), op, tol * tol);
     after_launch(P->ctx, "bk_scalars");
 }
 
@@ -2055,16 +2106,16 @@ static void batch_cycle(msbg_poisson* P, double* x64, const float* b, int K, dou
         seg_dot(P, p, q, S_PQ);
         scalars(P, 0, tol);
         begin_launch(ctx);
-        bk_add64<<<grid_for(n), 256, 0, ctx->stream>>>(n, lg3, bp, sc, p, x64);
+        launch_chained(ctx->stream, bk_add64, grid_for(n), 256, 0, 1, n, lg3, bp, sc, p, x64);
         after_launch(ctx, "bk_add64");
         begin_launch(ctx);
-        bk_axpy<<<grid_for(n), 256, 0, ctx->stream>>>(n, lg3, bp, sc, S_ALPHA, -1.0f, q, r);
+        launch_chained(ctx->stream, bk_axpy, grid_for(n), 256, 0, 1, n, lg3, bp, sc, S_ALPHA, -1.0f, q, r);
         after_launch(ctx, "bk_axpy");
         vcycle(P, 0, z, r, true);
         seg_dot(P, r, z, S_RZN);
         scalars(P, 1, tol);
         begin_launch(ctx);
-        bk_xpay<<<grid_for(n), 256, 0, ctx->stream>>>(n, lg3, bp, sc, z, p);
+        launch_chained(ctx->stream, bk_xpay, grid_for(n), 256, 0, 1, n, lg3, bp, sc, z, p);
         after_launch(ctx, "bk_xpay");
     }
     launch_residual64(P, x64, b, r);
@@ -2120,11 +2171,9 @@ static void autotune(msbg_poisson* P) {
             for (int c = 0; c < kNumShapes; ++c) {
                 auto run = [&]() {
                     if (kind == 0)
-                        pk_jacobi<<<shape_grid(c, cells), kShapes[c].threads, 0, ctx->stream>>>(
-                            level_args(L), L.x.as<float>(), L.b.as<float>(), L.t.as<float>(), P->omega);
+                        launch_chained(ctx->stream, pk_jacobi, shape_grid(c, cells), kShapes[c].threads, 0, 1, level_args(L), L.x.as<float>(), L.b.as<float>(), L.t.as<float>(), P->omega);
                     else
-                        pk_residual<<<shape_grid(c, cells), kShapes[c].threads, 0, ctx->stream>>>(
-                            level_args(L), L.x.as<float>(), L.b.as<float>(), L.r.as<float>());
+                        launch_chained(ctx->stream, pk_residual, shape_grid(c, cells), kShapes[c].threads, 0, 1, level_args(L), L.x.as<float>(), L.b.as<float>(), L.r.as<float>());
                 };
                 run();
                 CUDA_CHECK(cudaEventRecord(e0, ctx->stream));
