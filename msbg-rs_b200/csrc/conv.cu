@@ -1,5 +1,6 @@
 // conv.cu -- block-sparse 3x3x3 convolutions on tcgen05 (see conv.cuh).
 #include <algorithm>
+#include <type_traits>
 
 #include "conv.cuh"
 #include "tc.cuh"
@@ -451,6 +452,177 @@ __global__ void __launch_bounds__(128) conv3_wgrad_kernel(ConvLevel L, const uin
     if (!ok && tid == 0) atomicOr(status, 1);
 }
 
+// Weight gradient on 8^3 and 4^3 blocks from staged halos.  CTA (dx, part)
+// forms the nine taps of one x shift over a range of whole blocks: per block
+// it copies the input halo, shifted by dx so that its rows are BS cells, and
+// the block's output gradient into shared memory once (STAGES blocks in
+// flight), as 16-byte rows of 8 channels:
+//   A [z: BS + 2][channel chunk][y: BS + 2][x: BS],  B [chunk][cell].
+// Sixteen consecutive cells of a plane are then 256 contiguous bytes, one
+// K = 16 step, at any y shift; and the chunks of a plane and of the planes
+// after it follow at one stride, so one MMA of M = 128 rows takes 128 / CIN
+// dz shifts at once (rows beyond dz = 2 are computed on whatever lies there
+// and ignored).  Three warps issue the three dy shifts' MMAs, alternating
+// between two accumulators each where TMEM has room.
+// The kernel it replaces gathered every tap's operand from global memory
+// (27 reads of each input row, index arithmetic per 16 bytes, nothing in
+// flight over its barrier).  Weight gradient of 776 blocks (B200), 8^3 cells,
+// 32 -> 32 channels: 523 -> 79 us; 4^3, 64 -> 64: 191 -> 42 us.
+template <int LG, int CIN, int COUT>
+struct WgHalo {
+    static constexpr int BS = 1 << LG, H = BS + 2, PC = H * BS;  // cells of a staged plane
+    static constexpr int NCH = CIN / 8, NCO = COUT / 8, CELLS = BS * BS * BS;
+    static constexpr int A_BYTES = H * NCH * PC * 16, B_BYTES = NCO * CELLS * 16;
+    static constexpr int STAGES = LG == 2 ? 4 : 2;
+    static constexpr int OFF_B = STAGES * A_BYTES;
+    static constexpr int OFF_BAR = OFF_B + STAGES * B_BYTES;
+    static constexpr int BYTES = OFF_BAR + 64;
+    static constexpr int PPM = 128 / CIN;            // dz shifts of one MMA
+    static constexpr int NM = (3 + PPM - 1) / PPM;   // MMAs for the three
+    static constexpr int COLS1 = 3 * NM * COUT;      // accumulator columns of the CTA's taps
+    static constexpr int NACC = 2 * COLS1 <= 512 ? 2 : 1;
+    static constexpr int TCOLS = NACC * COLS1 <= 128 ? 128 : NACC * COLS1 <= 256 ? 256 : 512;
+    // the last M rows of the last planes read past the A stages
+    static constexpr int PAST = ((BS - 1 + (NM - 1) * PPM) * NCH + 16) * PC * 16 + 2 * BS * 16;
+    // More than half of the SM's shared memory: one CTA per SM, so the TMEM
+    // columns are never contended.
+    static constexpr int ALLOC = BYTES < 116 * 1024 ? 116 * 1024 : BYTES;
+    static constexpr bool FITS = ALLOC <= 227 * 1024 && PAST - A_BYTES <= STAGES * B_BYTES && COLS1 <= 512;
+};
+constexpr int kWgThreads = 256;
+
+template <int LG, int CIN, int COUT>
+__global__ void __launch_bounds__(kWgThreads) conv3_wgrad_halo_kernel(ConvLevel L, const uint16_t* __restrict__ x,
+                                                                      const uint16_t* __restrict__ dy, float* __restrict__ partial,
+                                                                      int* __restrict__ status) {
+    using S = WgHalo<LG, CIN, COUT>;
+    constexpr int BS = S::BS, H = S::H, PC = S::PC, NCH = S::NCH, ST = S::STAGES;
+    constexpr int MROWS = ((27 * CIN + 127) / 128) * 128;
+    constexpr int KSTEPS = S::CELLS / 16, KPP = BS * BS / 16;  // K steps of a block, of a plane
+    constexpr uint32_t IDESC = tc::idesc_bf16(128, COUT, 1, 1);
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::OFF_BAR);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + ST);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int dx = blockIdx.x, part = blockIdx.y;
+    const int64_t k0 = L.n_blocks * part / gridDim.y, k1 = L.n_blocks * (part + 1) / gridDim.y;
+    const int nblk = (int)(k1 - k0);
+    if (warp == 0) tc::tmem_alloc(tslot, S::TCOLS);
+    if (tid == 0) {
+        for (int s = 0; s < ST; ++s) tc::mbar_init(&bars[s], 3);  // one commit per issuing warp
+        tc::fence_mbar_init();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = *tslot;
+
+    // Block k0 + i into its stage.  Consecutive lanes take two chunks of
+    // eight cells: pairs of 16-byte pieces from one cell's row, written
+    // two to a bank group.
+    auto issue = [&](int i) {
+        const int64_t k = k0 + i;
+        uint8_t* ast = smem + (i % ST) * S::A_BYTES;
+        const int32_t* nbr = L.nbr27 + k * 27;
+#pragma unroll 4
+        for (int e = tid; e < H * NCH * PC; e += kWgThreads) {
+            const int g = (e >> 4) / (NCH / 2), j = ((e >> 4) % (NCH / 2)) * 2 + (e & 1);
+            const int p = (g % (PC / 8)) * 8 + ((e >> 1) & 7), z = g / (PC / 8);
+            const int lx = p % BS, ly = p / BS;
+            const int gx = lx + dx - 1, gy = ly - 1, gz = z - 1;
+            const int ox = gx < 0 ? 0 : (gx >= BS ? 2 : 1), oy = gy < 0 ? 0 : (gy >= BS ? 2 : 1), oz = gz < 0 ? 0 : (gz >= BS ? 2 : 1);
+            const int code = ox + 3 * oy + 9 * oz;
+            const int32_t kk = code == 13 ? (int32_t)k : __ldg(nbr + code);
+            const bool present = kk >= 0 && kk < L.n_blocks;
+            const int64_t c2 = present ? ((int64_t)kk << (3 * LG)) + ((gx & (BS - 1)) | ((gy & (BS - 1)) << LG) | ((gz & (BS - 1)) << (2 * LG))) : 0;
+            cp16_zfill(ast + ((z * NCH + j) * PC + p) * 16, reinterpret_cast<const uint4*>(x + c2 * CIN) + j, present);
+        }
+        uint8_t* bst = smem + S::OFF_B + (i % ST) * S::B_BYTES;
+        const uint4* src = reinterpret_cast<const uint4*>(dy + (k << (3 * LG)) * COUT);
+#pragma unroll 4
+        for (int e = tid; e < S::NCO * S::CELLS; e += kWgThreads) {
+            const int g = (e >> 4) / (S::NCO / 2), j = ((e >> 4) % (S::NCO / 2)) * 2 + (e & 1), c = g * 8 + ((e >> 1) & 7);
+            cp16_zfill(bst + (j * S::CELLS + c) * 16, src + c * S::NCO + j, true);
+        }
+    };
+#pragma unroll 1
+    for (int i = 0; i < ST - 1; ++i) {
+        if (i < nblk) issue(i);
+        cp_commit();
+    }
+    bool ok = true;
+#pragma unroll 1
+    for (int i = 0; i < nblk; ++i) {
+        const int nxt = i + ST - 1;
+        if (nxt < nblk) {
+            // the stage's previous block, i - 1: its MMAs have read it
+            if (i >= 1) ok &= tc::mbar_wait(&bars[nxt % ST], ((i - 1) / ST) & 1);
+            issue(nxt);
+        }
+        cp_commit();
+        cp_wait<ST - 1>();  // this thread's copies of block i have landed
+        tc::fence_async_smem();
+        __syncthreads();
+        if (lane == 0 && warp < 3) {
+            tc::fence_after_sync();
+            const uint32_t a0 = tc::smem_u32(smem + (i % ST) * S::A_BYTES) + (uint32_t)(warp * BS * 16);  // dy = warp
+            const uint32_t b0 = tc::smem_u32(smem + S::OFF_B + (i % ST) * S::B_BYTES);
+#pragma unroll 4
+            for (int kk = 0; kk < KSTEPS; ++kk) {
+                const int z = kk / KPP, acc = kk % S::NACC;
+                const uint64_t bd = tc::sdesc(b0 + (uint32_t)(kk * 256), 128, S::CELLS * 16);
+#pragma unroll
+                for (int nm = 0; nm < S::NM; ++nm) {
+                    const uint64_t ad = tc::sdesc(a0 + (uint32_t)((z + nm * S::PPM) * NCH * PC * 16 + (kk % KPP) * 256), 128, PC * 16);
+                    tc::mma_bf16(tmem + (uint32_t)(((acc * 3 + warp) * S::NM + nm) * COUT), ad, bd, IDESC, i > 0 || kk >= S::NACC);
+                }
+            }
+            tc::mma_commit(&bars[i % ST]);
+        }
+    }
+    if (nblk > 0) {
+        ok &= tc::mbar_wait(&bars[(nblk - 1) % ST], ((nblk - 1) / ST) & 1);
+        tc::fence_after_sync();
+    }
+    if (warp < 4) {
+        __syncwarp();  // tcgen05.ld is warp-wide
+        const int m = tid;  // row: dz shift m / CIN of its MMA, input channel m % CIN
+#pragma unroll 1
+        for (int d = 0; d < 3; ++d) {
+#pragma unroll 1
+            for (int nm = 0; nm < S::NM; ++nm) {
+                const int dz = nm * S::PPM + m / CIN;
+                float* out = partial + ((int64_t)part * MROWS + (dx + 3 * d + 9 * dz) * CIN + m % CIN) * COUT;
+#pragma unroll 1
+                for (int c0 = 0; c0 < COUT; c0 += 16) {
+                    float v[16];
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) v[q] = 0.0f;
+                    if (nblk > 0) {
+                        float t[16];
+                        tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((d * S::NM + nm) * COUT + c0), v);
+                        if (S::NACC == 2) {
+                            tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(((3 + d) * S::NM + nm) * COUT + c0), t);
+#pragma unroll
+                            for (int q = 0; q < 16; ++q) v[q] += t[q];
+                        }
+                    }
+                    if (dz < 3) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            reinterpret_cast<float4*>(out + c0)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    }
+                }
+            }
+        }
+    }
+    cp_wait<0>();
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, S::TCOLS);
+    if (!ok && tid == 0) atomicOr(status, 1);
+}
+
 // dw[t][o][i] (+)= sum over parts (in order) of partial[part][t * CIN + i][o]
 __global__ void conv3_wgrad_reduce_kernel(const float* __restrict__ partial, int parts, int cin, int cout, int mrows,
                                           float* __restrict__ dw, int acc) {
@@ -511,6 +683,37 @@ static void launch_wgrad(msbg_ctx* ctx, const ConvLevel& L, const uint16_t* x, c
     constexpr int MT = (27 * CIN + 127) / 128;
     constexpr int MROWS = MT * 128;
     const int64_t cells = L.cells();
+    // 8^3 and 4^3 blocks whose stages fit shared memory: from staged halos,
+    // one CTA per SM over the three x shifts
+    auto from_halos = [&](auto lg) {
+        constexpr int LG = decltype(lg)::value;
+        using W = WgHalo<LG, CIN, COUT>;
+        if constexpr (W::FITS) {
+            static bool wattr = false;
+            if (!wattr) {
+                CUDA_CHECK(cudaFuncSetAttribute(conv3_wgrad_halo_kernel<LG, CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                W::ALLOC));
+                wattr = true;
+            }
+            const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(L.n_blocks, 148 / 3));
+            ScratchLayout SL;
+            const size_t op = SL.add<float>((size_t)parts * MROWS * COUT);
+            float* partial = ScratchLayout::at<float>(scratch(ctx, SL), op);
+            begin_launch(ctx);
+            conv3_wgrad_halo_kernel<LG, CIN, COUT><<<dim3(3, (unsigned)parts), kWgThreads, W::ALLOC, ctx->stream>>>(
+                L, x, dy, partial, ctx->status.as<int>());
+            after_launch(ctx, "conv3_wgrad_halo_kernel");
+            begin_launch(ctx);
+            conv3_wgrad_reduce_kernel<<<(27 * CIN * COUT + 255) / 256, 256, 0, ctx->stream>>>(partial, parts, CIN, COUT, MROWS, dw,
+                                                                                               acc ? 1 : 0);
+            after_launch(ctx, "conv3_wgrad_reduce_kernel");
+            return true;
+        } else {
+            return false;
+        }
+    };
+    if (L.lg == 3 && from_halos(std::integral_constant<int, 3>())) return;
+    if (L.lg == 2 && from_halos(std::integral_constant<int, 2>())) return;
     // about 4 CTAs per SM in total, each over a contiguous range of whole 64-cell chunks
     const int64_t chunks = std::max<int64_t>(1, (cells + kWgCells - 1) / kWgCells);
     const int parts = (int)std::min<int64_t>(chunks, std::max<int64_t>(1, 592 / MT));

@@ -1,0 +1,32 @@
+"""The weight gradient from staged halos: one block to more than the CTAs take
+one each, every channel pair whose stages fit, isolated and touching blocks;
+within the f32 accumulation bound of the FP64 oracle (as
+tests/test_gpu_conv.py)."""
+import numpy as np
+import pytest
+
+from test_gpu_conv import dev_bits, level
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nb,frac", [(1, 1.0), (2, 0.4), (5, 0.9), (7, 0.6)])
+@pytest.mark.parametrize("lg,cin,cout", [(2, 16, 16), (2, 32, 32), (2, 64, 64), (2, 64, 16), (2, 16, 64), (3, 16, 16),
+                                         (3, 32, 32), (3, 16, 32)])
+def test_wgrad_from_halos(msbg, ctx, nb, frac, lg, cin, cout):
+    import torch
+    unet, act, nbr, taps = level(nb, lg, frac, seed=nb + 3 * lg + cin)
+    cells = len(act) << (3 * lg)
+    rng = np.random.default_rng(nb * cin + cout)
+    xb = unet.bf16_bits(rng.standard_normal((cells, cin)).astype(np.float32))
+    gb = unet.bf16_bits(rng.standard_normal((cells, cout)).astype(np.float32))
+    x, g = unet.bf16_value(xb), unet.bf16_value(gb)
+    ref = unet.conv3_wgrad(x, g, taps)
+    absum = unet.conv3_wgrad(np.abs(x), np.abs(g), taps)
+    d_nbr = torch.from_numpy(nbr).cuda()
+    d_x, d_g = dev_bits(xb), dev_bits(gb)
+    dw = torch.empty((27, cout, cin), dtype=torch.float32, device="cuda")
+    ptr = msbg._lib.ptr
+    torch.cuda.synchronize()
+    msbg._lib.call("msbg_conv3_wgrad_device", ctx.handle, ptr(d_nbr), len(act), lg, cin, cout, ptr(d_x), ptr(d_g), ptr(dw))
+    assert np.all(np.abs(dw.cpu().numpy() - ref) <= 1e-5 * absum + 1e-30)
