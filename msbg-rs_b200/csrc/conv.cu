@@ -345,6 +345,216 @@ __global__ void __launch_bounds__(kB8Threads) conv3_b8_kernel(ConvLevel L, const
     if (!ok && tid == 0) atomicOr(status, 1);
 }
 
+// Copies the input halo of block k, shifted by dx so that its rows are BS
+// cells, into shared memory as 16-byte rows of 8 channels: chunk j of the
+// cell at halo row (z, y) and column lx goes to
+// dst + j * CS + z * ZS + (y * BS + lx) * 16 (zeros outside the active blocks).
+// A warp takes a whole row of cells and chunks at a time (or several): the
+// row's neighbour blocks come from a lane's register by a shuffle and the
+// address is a row base plus a lane constant, about a dozen instructions per
+// 32 pieces (worked out per piece they bound the kernels below).  Consecutive
+// lanes take pairs of chunks of one cell (a sector); CS is 64 bytes past a
+// multiple of 128, so the pairs fall on different banks.
+template <int LG, int CIN, int NT, int CS, int ZS>
+__device__ __forceinline__ void stage_halo(const ConvLevel& L, const uint16_t* __restrict__ x, int64_t k, int dx, uint8_t* dst) {
+    constexpr int BS = 1 << LG, H = BS + 2, NCH = CIN / 8, M = BS - 1;
+    constexpr int IPR = BS * NCH;                        // pieces of a row
+    constexpr int RPI = IPR < 32 ? 32 / IPR : 1;         // rows a warp takes at once
+    constexpr int IPL = IPR > 32 ? IPR / 32 : 1;         // pieces of a row per lane
+    static_assert(CS % 128 == 64, "chunk pairs must fall on different banks");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int32_t nb = lane == 13 ? (int32_t)k : lane < 27 ? __ldg(L.nbr27 + k * 27 + lane) : -1;
+    const int within = lane % (IPR < 32 ? IPR : 32), sub = lane / (IPR < 32 ? IPR : 32);
+#pragma unroll
+    for (int h = 0; h < IPL; ++h) {
+        const int q = within + 32 * h;
+        const int j = (q >> 1) / BS * 2 + (q & 1), lx = (q >> 1) % BS;
+        const int gx = lx + dx - 1, ox = gx < 0 ? 0 : (gx >= BS ? 2 : 1);
+        const uint16_t* xl = x + (gx & M) * CIN + j * 8;
+        uint8_t* dl = dst + j * CS + lx * 16;
+#pragma unroll 4
+        for (int r0 = warp * RPI; r0 < H * H; r0 += NT / 32 * RPI) {
+            const int r = RPI == 1 ? r0 : min(r0 + sub, H * H - 1);  // (a row past the last repeats it)
+            const int z = r / H, y = r - z * H;
+            const int oy = y == 0 ? 0 : (y == H - 1 ? 2 : 1), oz = z == 0 ? 0 : (z == H - 1 ? 2 : 1);
+            const int32_t kk = __shfl_sync(0xffffffffu, nb, ox + 3 * oy + 9 * oz);
+            const bool present = kk >= 0 && kk < L.n_blocks;
+            const uint32_t cell = ((uint32_t)((y - 1) & M) << LG) | ((uint32_t)((z - 1) & M) << (2 * LG));
+            const uint16_t* src = present ? xl + (((int64_t)kk << (3 * LG)) + cell) * CIN : x;
+            cp16_zfill(dl + z * ZS + y * (BS * 16), src, present);
+        }
+    }
+}
+
+// 4^3 blocks from staged halos: persistent CTAs, one per SM, over the blocks.
+// The work is cut into units (x shift dx, block): the block's input halo
+// shifted by dx, so that its rows are BS cells, is copied into one of two
+// buffers as 16-byte rows of 8 channels,
+//   A [channel chunk][z: BS + 2][y: BS + 2][x: BS].
+// The operand of tap (dx, dy, dz) for 128 consecutive rows of the padded plane
+// order (z, y of BS + 2, x) is then one contiguous, 16-byte-row view at any
+// (dy, dz) shift, so a unit's nine taps need no staging of their own; rows
+// with y >= BS (and past the last plane) are computed on whatever lies there
+// and ignored.  The nine taps' weights of one dx are in shared memory at a
+// time (double-buffered), taken for up to 8 blocks whose accumulators stay in
+// TMEM over the three dx.  776 blocks, 64 -> 64 channels (B200): 94 us with
+// every tap's rows gathered from global memory, 61 us.  (8^3 blocks run five
+// such tiles per block and read shared memory as fast, but copy their halo
+// three times: 84 us against 69 us for conv3_b8_kernel, 32 -> 32 channels.)
+constexpr int kHaloThreads = 512;
+
+template <int CIN, int COUT>
+struct FwdHalo {
+    static constexpr int LG = 2, BS = 1 << LG, H = BS + 2, PC = H * BS;
+    static constexpr int NCH = CIN / 8, CS = (H * PC * 16) / 128 * 128 + 64 + (H * PC * 16 % 128 > 64 ? 128 : 0);  // bytes of a chunk
+    static constexpr int A_BYTES = NCH * CS;
+    static constexpr int STAGES = 2;
+    static constexpr int W_TAP = COUT * CIN * 2;
+    static constexpr int W_BYTES = 2 * 9 * W_TAP;
+    static constexpr int GROUP = 8;  // blocks per pass over dx, an accumulator of COUT columns each
+    static constexpr int TCOLS = GROUP * COUT;
+    static constexpr int OFF_W = STAGES * A_BYTES;
+    static constexpr int OFF_BAR = OFF_W + W_BYTES;
+    static constexpr int BYTES = OFF_BAR + 64;
+    // More than half of the SM's shared memory: one CTA per SM, so the
+    // TMEM columns are never contended.
+    static constexpr int ALLOC = BYTES < 116 * 1024 ? 116 * 1024 : BYTES;
+    static_assert(BS * PC <= 128, "a block's padded cells are the rows of one MMA");
+    static_assert(ALLOC <= 227 * 1024 && TCOLS <= 512, "stages or accumulators too large");
+    // the last rows of the tile read past their chunk
+    static_assert((2 * PC + 2 * BS + 128) * 16 - CS <= W_BYTES, "operand rows past the stages");
+};
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kHaloThreads) conv3_halo_kernel(ConvLevel L, const uint16_t* __restrict__ x,
+                                                                  const uint16_t* __restrict__ w,
+                                                                  const float* __restrict__ bias, int relu,
+                                                                  const uint16_t* __restrict__ mask, int out_f32, int out_ch,
+                                                                  void* __restrict__ y, int* __restrict__ status) {
+    using S = FwdHalo<CIN, COUT>;
+    constexpr int LG = S::LG, BS = S::BS, H = S::H, PC = S::PC, NCH = S::NCH, ST = S::STAGES;
+    constexpr uint32_t SBO_W = NCH * 128;
+    constexpr uint32_t IDESC = tc::idesc_bf16(128, COUT, 0, 0);
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::OFF_BAR);
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + ST);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // this CTA's blocks k0 .. k0 + nblk - 1, in groups of GROUP; unit u of a
+    // group of g blocks is (dx = u / g, block u % g)
+    const int64_t k0 = L.n_blocks * blockIdx.x / gridDim.x, k1 = L.n_blocks * (blockIdx.x + 1) / gridDim.x;
+    const int nblk = (int)(k1 - k0), units = 3 * nblk;
+    if (warp == 0) tc::tmem_alloc(tslot, S::TCOLS);
+    if (tid == 0) {
+        for (int s = 0; s < ST; ++s) tc::mbar_init(&bars[s], 1);
+        tc::fence_mbar_init();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = *tslot;
+
+    struct Unit {
+        int block, dx, slot;     // block of the CTA, x shift, accumulator
+        int pass;                // passes over dx before this one, 3 per group
+        bool group_first, group_last;  // first block of its pass, last unit of its group
+    };
+    auto unit = [&](int u) {
+        Unit r;
+        const int gi = u / (3 * S::GROUP), v = u - gi * 3 * S::GROUP;
+        const int b0 = gi * S::GROUP, g = min(S::GROUP, nblk - b0);
+        r.dx = v / g;
+        const int b = v - r.dx * g;
+        r.block = b0 + b;
+        r.slot = b;
+        r.pass = 3 * gi + r.dx;
+        r.group_first = b == 0;
+        r.group_last = v == 3 * g - 1;
+        return r;
+    };
+    auto issue = [&](int u) {
+        const Unit r = unit(u);
+        const int64_t k = k0 + r.block;
+        uint8_t* ast = smem + (u % ST) * S::A_BYTES;
+        stage_halo<LG, CIN, kHaloThreads, S::CS, PC * 16>(L, x, k, r.dx, ast);
+        // the pass's weights, taps dx + 3 i (the MMAs of the pass before last,
+        // whose buffer this is, are done: so are those of unit u - 2)
+        if (r.group_first) {
+            uint8_t* wst = smem + S::OFF_W + (r.pass & 1) * 9 * S::W_TAP;
+            for (int e = tid; e < 9 * COUT * NCH; e += kHaloThreads) {
+                const int t = e / (COUT * NCH), q = e % (COUT * NCH), o = q / NCH, j = q % NCH;
+                cp16_zfill(wst + t * S::W_TAP + (o >> 3) * SBO_W + j * 128 + (o & 7) * 16,
+                           reinterpret_cast<const uint4*>(w) + (int64_t)(r.dx + 3 * t) * (COUT * NCH) + q, true);
+            }
+        }
+    };
+    // row m of the tile is padded cell m; four warps write a block
+    auto epilogue = [&](int block, int slot) {
+        __syncwarp();  // tcgen05.ld is warp-wide
+        float acc[16];
+        const int q = (warp & 3) * 32 + lane;
+        const int cx = q % BS, cy = (q / BS) % H, cz = q / PC;
+        const bool valid = cy < BS && cz < BS;
+        const int64_t cell = ((k0 + block) << (3 * LG)) + (valid ? cx | (cy << LG) | (cz << (2 * LG)) : 0);
+#pragma unroll
+        for (int c0 = 0; c0 < COUT; c0 += 16) {
+            tc::tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(slot * COUT + c0), acc);
+            if (valid && c0 < out_ch) store16<COUT>(acc, cell, c0, bias, relu, mask, out_f32, out_ch, y);
+        }
+    };
+#pragma unroll 1
+    for (int u = 0; u < ST - 1; ++u) {
+        if (u < units) issue(u);
+        cp_commit();
+    }
+    bool ok = true;
+#pragma unroll 1
+    for (int u = 0; u < units; ++u) {
+        cp_wait<ST - 2>();  // this thread's copies of unit u have landed
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        __syncthreads();
+        const Unit r = unit(u);
+        if (tid == 0) {
+            tc::fence_after_sync();
+            const uint64_t a0 = tc::sdesc(tc::smem_u32(smem + (u % ST) * S::A_BYTES), S::CS, 128);
+            const uint64_t b0 = tc::sdesc(tc::smem_u32(smem + S::OFF_W + (r.pass & 1) * 9 * S::W_TAP), 128, SBO_W);
+            const uint32_t d = tmem + (uint32_t)(r.slot * COUT);
+#pragma unroll 1
+            for (int dz = 0; dz < 3; ++dz) {
+#pragma unroll
+                for (int dy = 0; dy < 3; ++dy) {
+#pragma unroll
+                    for (int kk = 0; kk < CIN / 16; ++kk) {
+                        // offsets in the 16-byte units of the descriptors' address field
+                        const uint64_t ao = (uint64_t)(dz * PC + dy * BS) + (uint64_t)((2 * kk * S::CS) >> 4);
+                        const uint64_t bo = (uint64_t)(((3 * dz + dy) * S::W_TAP + kk * 256) >> 4);
+                        tc::mma_bf16(d, a0 + ao, b0 + bo, IDESC, (r.dx | dz | dy | kk) != 0);
+                    }
+                }
+            }
+            tc::mma_commit(&bars[u % ST]);
+        }
+        // with this unit's MMAs queued, the stage of the unit before (whose
+        // MMAs have then read it) is filled again
+        const int nxt = u + ST - 1;
+        if (nxt < units) {
+            if (u >= 1) ok &= tc::mbar_wait(&bars[nxt % ST], ((u - 1) / ST) & 1);
+            issue(nxt);
+        }
+        cp_commit();
+        if (r.group_last) {  // the group's blocks, a set of four warps each
+            ok &= tc::mbar_wait(&bars[u % ST], (u / ST) & 1);
+            tc::fence_after_sync();
+            for (int b = warp >> 2; b <= r.slot; b += kHaloThreads / 128) epilogue(r.block - r.slot + b, b);
+        }
+    }
+    cp_wait<0>();
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, S::TCOLS);
+    if (!ok && tid == 0) atomicOr(status, 1);
+}
+
 template <int CIN, int COUT>
 struct WgSmem {
     static constexpr int A_BYTES = 128 * kWgCells * 2;
@@ -472,7 +682,8 @@ template <int LG, int CIN, int COUT>
 struct WgHalo {
     static constexpr int BS = 1 << LG, H = BS + 2, PC = H * BS;  // cells of a staged plane
     static constexpr int NCH = CIN / 8, NCO = COUT / 8, CELLS = BS * BS * BS;
-    static constexpr int A_BYTES = H * NCH * PC * 16, B_BYTES = NCO * CELLS * 16;
+    static constexpr int CS = PC * 16 / 128 * 128 + 64 + (PC * 16 % 128 > 64 ? 128 : 0);  // bytes of a chunk of a plane
+    static constexpr int A_BYTES = H * NCH * CS, B_BYTES = NCO * CELLS * 16;
     static constexpr int STAGES = LG == 2 ? 4 : 2;
     static constexpr int OFF_B = STAGES * A_BYTES;
     static constexpr int OFF_BAR = OFF_B + STAGES * B_BYTES;
@@ -483,20 +694,20 @@ struct WgHalo {
     static constexpr int NACC = 2 * COLS1 <= 512 ? 2 : 1;
     static constexpr int TCOLS = NACC * COLS1 <= 128 ? 128 : NACC * COLS1 <= 256 ? 256 : 512;
     // the last M rows of the last planes read past the A stages
-    static constexpr int PAST = ((BS - 1 + (NM - 1) * PPM) * NCH + 16) * PC * 16 + 2 * BS * 16;
+    static constexpr int PAST = ((BS - 1 + (NM - 1) * PPM) * NCH + 16) * CS + 2 * BS * 16;
     // More than half of the SM's shared memory: one CTA per SM, so the TMEM
     // columns are never contended.
     static constexpr int ALLOC = BYTES < 116 * 1024 ? 116 * 1024 : BYTES;
     static constexpr bool FITS = ALLOC <= 227 * 1024 && PAST - A_BYTES <= STAGES * B_BYTES && COLS1 <= 512;
 };
-constexpr int kWgThreads = 256;
+constexpr int kWgThreads = 512;
 
 template <int LG, int CIN, int COUT>
 __global__ void __launch_bounds__(kWgThreads) conv3_wgrad_halo_kernel(ConvLevel L, const uint16_t* __restrict__ x,
                                                                       const uint16_t* __restrict__ dy, float* __restrict__ partial,
                                                                       int* __restrict__ status) {
     using S = WgHalo<LG, CIN, COUT>;
-    constexpr int BS = S::BS, H = S::H, PC = S::PC, NCH = S::NCH, ST = S::STAGES;
+    constexpr int BS = S::BS, NCH = S::NCH, ST = S::STAGES;
     constexpr int MROWS = ((27 * CIN + 127) / 128) * 128;
     constexpr int KSTEPS = S::CELLS / 16, KPP = BS * BS / 16;  // K steps of a block, of a plane
     constexpr uint32_t IDESC = tc::idesc_bf16(128, COUT, 1, 1);
@@ -517,26 +728,10 @@ __global__ void __launch_bounds__(kWgThreads) conv3_wgrad_halo_kernel(ConvLevel 
     tc::fence_after_sync();
     const uint32_t tmem = *tslot;
 
-    // Block k0 + i into its stage.  Consecutive lanes take two chunks of
-    // eight cells: pairs of 16-byte pieces from one cell's row, written
-    // two to a bank group.
+    // Block k0 + i into its stage
     auto issue = [&](int i) {
         const int64_t k = k0 + i;
-        uint8_t* ast = smem + (i % ST) * S::A_BYTES;
-        const int32_t* nbr = L.nbr27 + k * 27;
-#pragma unroll 4
-        for (int e = tid; e < H * NCH * PC; e += kWgThreads) {
-            const int g = (e >> 4) / (NCH / 2), j = ((e >> 4) % (NCH / 2)) * 2 + (e & 1);
-            const int p = (g % (PC / 8)) * 8 + ((e >> 1) & 7), z = g / (PC / 8);
-            const int lx = p % BS, ly = p / BS;
-            const int gx = lx + dx - 1, gy = ly - 1, gz = z - 1;
-            const int ox = gx < 0 ? 0 : (gx >= BS ? 2 : 1), oy = gy < 0 ? 0 : (gy >= BS ? 2 : 1), oz = gz < 0 ? 0 : (gz >= BS ? 2 : 1);
-            const int code = ox + 3 * oy + 9 * oz;
-            const int32_t kk = code == 13 ? (int32_t)k : __ldg(nbr + code);
-            const bool present = kk >= 0 && kk < L.n_blocks;
-            const int64_t c2 = present ? ((int64_t)kk << (3 * LG)) + ((gx & (BS - 1)) | ((gy & (BS - 1)) << LG) | ((gz & (BS - 1)) << (2 * LG))) : 0;
-            cp16_zfill(ast + ((z * NCH + j) * PC + p) * 16, reinterpret_cast<const uint4*>(x + c2 * CIN) + j, present);
-        }
+        stage_halo<LG, CIN, kWgThreads, S::CS, NCH * S::CS>(L, x, k, dx, smem + (i % ST) * S::A_BYTES);
         uint8_t* bst = smem + S::OFF_B + (i % ST) * S::B_BYTES;
         const uint4* src = reinterpret_cast<const uint4*>(dy + (k << (3 * LG)) * COUT);
 #pragma unroll 4
@@ -553,14 +748,7 @@ __global__ void __launch_bounds__(kWgThreads) conv3_wgrad_halo_kernel(ConvLevel 
     bool ok = true;
 #pragma unroll 1
     for (int i = 0; i < nblk; ++i) {
-        const int nxt = i + ST - 1;
-        if (nxt < nblk) {
-            // the stage's previous block, i - 1: its MMAs have read it
-            if (i >= 1) ok &= tc::mbar_wait(&bars[nxt % ST], ((i - 1) / ST) & 1);
-            issue(nxt);
-        }
-        cp_commit();
-        cp_wait<ST - 1>();  // this thread's copies of block i have landed
+        cp_wait<ST - 2>();  // this thread's copies of block i have landed
         tc::fence_async_smem();
         __syncthreads();
         if (lane == 0 && warp < 3) {
@@ -573,12 +761,20 @@ __global__ void __launch_bounds__(kWgThreads) conv3_wgrad_halo_kernel(ConvLevel 
                 const uint64_t bd = tc::sdesc(b0 + (uint32_t)(kk * 256), 128, S::CELLS * 16);
 #pragma unroll
                 for (int nm = 0; nm < S::NM; ++nm) {
-                    const uint64_t ad = tc::sdesc(a0 + (uint32_t)((z + nm * S::PPM) * NCH * PC * 16 + (kk % KPP) * 256), 128, PC * 16);
+                    const uint64_t ad = tc::sdesc(a0 + (uint32_t)((z + nm * S::PPM) * NCH * S::CS + (kk % KPP) * 256), 128, S::CS);
                     tc::mma_bf16(tmem + (uint32_t)(((acc * 3 + warp) * S::NM + nm) * COUT), ad, bd, IDESC, i > 0 || kk >= S::NACC);
                 }
             }
             tc::mma_commit(&bars[i % ST]);
         }
+        // with this block's MMAs queued, the stage of the block before (whose
+        // MMAs have then read it) is filled again
+        const int nxt = i + ST - 1;
+        if (nxt < nblk) {
+            if (i >= 1) ok &= tc::mbar_wait(&bars[nxt % ST], ((i - 1) / ST) & 1);
+            issue(nxt);
+        }
+        cp_commit();
     }
     if (nblk > 0) {
         ok &= tc::mbar_wait(&bars[(nblk - 1) % ST], ((nblk - 1) / ST) & 1);
@@ -665,6 +861,21 @@ static void launch_fwd(msbg_ctx* ctx, const ConvLevel& L, const uint16_t* x, con
             after_launch(ctx, "conv3_b8_kernel");
             return;
         }
+    }
+    if (L.lg == 2) {
+        using H = FwdHalo<CIN, COUT>;
+        static bool hattr = false;
+        if (!hattr) {
+            CUDA_CHECK(cudaFuncSetAttribute(conv3_halo_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, H::ALLOC));
+            hattr = true;
+        }
+        static int sms = 0;
+        if (!sms) CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+        begin_launch(ctx);
+        conv3_halo_kernel<CIN, COUT><<<(unsigned)std::min<int64_t>(L.n_blocks, sms), kHaloThreads, H::ALLOC, ctx->stream>>>(
+            L, x, w, bias, relu ? 1 : 0, mask, out_f32 ? 1 : 0, out_ch > 0 ? out_ch : COUT, y, ctx->status.as<int>());
+        after_launch(ctx, "conv3_halo_kernel");
+        return;
     }
     begin_launch(ctx);
     conv3_fwd_kernel<CIN, COUT><<<(unsigned)((cells + 127) / 128), 128, S::ALLOC, ctx->stream>>>(

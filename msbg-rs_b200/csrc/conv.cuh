@@ -16,16 +16,19 @@
 // shared memory once (double-buffered) and the weights of all taps once;
 // every tap's operand for one z-plane of the block is a strided view of the
 // halo, so the MMAs (M = 64 cells of a plane) need no per-tap staging, and
-// eight warps issue the eight planes' MMAs side by side.  Other shapes run as
+// eight warps issue the eight planes' MMAs side by side.  On 4^3 blocks they
+// run as conv3_halo_kernel, which copies each block's halo once per x shift
+// and takes that shift's nine taps as views of it.  Other shapes run as
 // conv3_fwd_kernel: one CTA computes a tile of 128 output cells x Cout in
 // TMEM; per tap its threads gather the shifted input rows (cp.async,
 // several taps in flight) into a K-major operand and the weights into a
 // K-major operand in shared memory, one thread issues Cin/16 MMAs and
 // commits them to the stage's mbarrier.  The weight gradient
 //   dw[t][o][i] = sum_c x[c + d(t)][i] dy[c][o]
-// runs as conv3_wgrad_kernel: M = the (tap, Cin) pairs in tiles of 128,
-// N = Cout, K = cells, operands MN-major (16-byte rows of 8 channels of one
-// cell), partial sums per cell range reduced in a fixed order.
+// runs with M = (tap, Cin) pairs, N = Cout, K = cells, operands MN-major
+// (16-byte rows of 8 channels of one cell), partial sums per cell range
+// reduced in a fixed order: as conv3_wgrad_halo_kernel from staged halos on
+// 8^3 and 4^3 blocks, as conv3_wgrad_kernel with gathered operands elsewhere.
 #pragma once
 
 #include "common.cuh"
