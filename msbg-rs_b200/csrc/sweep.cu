@@ -273,6 +273,220 @@ __device__ __forceinline__ void sweep_compute(const SweepArgs& a, const float* _
     }
 }
 
+// Pairs of f32 in one 64-bit register and the paired IEEE single-precision
+// operations of sm_100 (each half rounded as the scalar operation).  The
+// stencils below feed no paired product directly into a paired sum (the
+// code generator may fuse such a pair even with .rn): products that feed sums
+// are scalar, the others go to explicit fused multiply-adds, as in the scalar
+// form.
+__device__ __forceinline__ uint64_t sw_pack(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void sw_unpack(uint64_t v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t sw_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t sw_sub(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t sw_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t sw_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t sw_ld2(const float* p) { return *reinterpret_cast<const uint64_t*>(p); }
+
+// Stores two x-neighbouring elements (x even).
+template <class T> __device__ __forceinline__ void store2(T* p, T a, T b);
+template <> __device__ __forceinline__ void store2<float>(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+template <> __device__ __forceinline__ void store2<uint16_t>(uint16_t* p, uint16_t a, uint16_t b) {
+    *reinterpret_cast<uint32_t*>(p) = (uint32_t)a | ((uint32_t)b << 16);
+}
+template <> __device__ __forceinline__ void store2<uint8_t>(uint8_t* p, uint8_t a, uint8_t b) {
+    *reinterpret_cast<uint16_t*>(p) = (uint16_t)(a | (b << 8));
+}
+
+// The stencil over one staged block, two x-columns and ZP planes per thread:
+// thread (xp, y, zi) walks columns x = 2 xp and x + 1 over its planes with
+// paired arithmetic, the same operations in the same order per cell as
+// sweep_compute, the taps of neighbouring planes sliding through registers.
+// For the pair, L = x - 1, AB = (x, x + 1) and R = x + 2 of a row give the
+// x-neighbour pairs (L, A) and (B, R).  Bound by issue: 25 taps in 13 loads and
+// about half the arithmetic per cell of one column per thread with every tap
+// loaded (10 sweeps of 4,688 bf16 blocks, B200: 1.04 -> 0.98 ms; 5 19-tap
+// sweeps of u16: 0.62 -> 0.48 ms).
+template <class E, int BSX, int ST, int ZP>
+__device__ __forceinline__ void sweep_compute_pair(const SweepArgs& a, const float* __restrict__ h, int slot, int pi, int tid) {
+    constexpr int HALO = ST == MSBG_BILAPLACIAN ? 2 : 1;
+    constexpr int HSX = BSX + 2 * HALO;
+    constexpr int RS = Stage<BSX>::RS;
+    constexpr int PL = HSX * RS;
+    constexpr int X0 = 4 - HALO;
+    constexpr int N = BSX * BSX * BSX, P2 = BSX * BSX, XP = BSX / 2;
+    constexpr int XD = ST == MSBG_BILAPLACIAN ? 2 : 1;
+    using T = typename E::T;
+    const int zi = tid / (XP * BSX), t = tid % (XP * BSX);
+    // 16^3 blocks: eight lanes a row; a half-warp takes rows y and y + 2,
+    // which fall on disjoint banks at this row pitch (24 floats)
+    const int x = 2 * (t % XP), yl = t / XP;
+    const int y = BSX == 16 ? (yl & ~3) | ((yl & 1) << 1) | ((yl >> 1) & 1) : yl;
+    const int z0 = zi * ZP, z1 = z0 + ZP;
+    T* out = (T*)a.payload + (size_t)slot * N + x + y * BSX;
+    // the side buffer's planes of the block's outer columns
+    float* xo = nullptr;
+    if (x < XD) xo = a.xface + ((size_t)slot * 2 * XD + x) * P2 + y;                     // A: x = 0, B: 1 (25 taps)
+    else if (x + 1 >= BSX - XD) xo = a.xface + ((size_t)slot * 2 * XD + XD) * P2 + y;   // B: x = BSX - 1, A: BSX - 2 (25 taps)
+    const bool lowside = x < XD;
+    const int i0 = (HALO * HSX + (y + HALO)) * RS + X0 + x + HALO;  // z = 0, column x
+    const float dt = a.dt;
+    const int clamp01 = a.clamp01;
+    uint32_t sa = 0, sb = 0, zs = 0;  // generator states of columns x and x + 1
+    if constexpr (std::is_same<E, ElemU8>::value) {
+        const uint64_t base = a.sr_base + (uint64_t)pi * (uint64_t)(N >> a.sr_lg) + 1;
+        const int e = x + y * BSX + z0 * P2, m = (1 << a.sr_lg) - 1;
+        const uint32_t pw = sr_pow(base + (uint64_t)(e >> a.sr_lg));  // x is even: both columns in one chunk
+        sa = a.sr_seed[x & m] * pw;
+        sb = a.sr_seed[(x + 1) & m] * pw;
+        zs = a.sr_zstep;
+    }
+    auto lo = [](uint64_t v) { float p, q; sw_unpack(v, p, q); return p; };
+    auto hi = [](uint64_t v) { float p, q; sw_unpack(v, p, q); return q; };
+    auto put = [&](int z, float n0, float n1) {
+        if (clamp01) {
+            n0 = clampf(n0, 0.0f, 1.0f);
+            n1 = clampf(n1, 0.0f, 1.0f);
+        }
+        const T va = StoreBack<E>::store(n0, sa), vb = StoreBack<E>::store(n1, sb);
+        sa *= zs;
+        sb *= zs;
+        store2<T>(out + z * P2, va, vb);
+        if (xo) {
+            if (XD == 2) {
+                xo[z * BSX] = E::load(lowside ? va : vb);
+                xo[P2 + z * BSX] = E::load(lowside ? vb : va);
+            } else {
+                xo[z * BSX] = E::load(lowside ? va : vb);
+            }
+        }
+    };
+    const uint64_t half2 = sw_pack(0.5f, 0.5f), dt2 = sw_pack(dt, dt);
+    const float* c0p = h + i0;
+    if (ST == MSBG_LAPLACIAN) {
+        const uint64_t m6 = sw_pack(-6.0f, -6.0f);
+        uint64_t zb = sw_ld2(c0p + (z0 - 1) * PL), c = sw_ld2(c0p + z0 * PL), zf = sw_ld2(c0p + (z0 + 1) * PL);
+#pragma unroll 4
+        for (int z = z0; z < z1; ++z) {
+            const float* p = c0p + z * PL;
+            const uint64_t lx = sw_pack(p[-1], lo(c)), rx = sw_pack(hi(c), p[2]);
+            const uint64_t dyu = sw_ld2(p - RS), dyd = sw_ld2(p + RS);
+            uint64_t nbs = sw_add(lx, rx);
+            nbs = sw_add(nbs, dyu);
+            nbs = sw_add(nbs, dyd);
+            nbs = sw_add(nbs, zb);
+            nbs = sw_add(nbs, zf);
+            const uint64_t lap = sw_fma(c, m6, nbs);
+            const uint64_t fx = sw_mul(sw_sub(rx, lx), half2), fy = sw_mul(sw_sub(dyd, dyu), half2), fz = sw_mul(sw_sub(zf, zb), half2);
+            float s0, s1, n0, n1;
+            sw_unpack(sw_fma(fx, fx, sw_fma(fy, fy, sw_mul(fz, fz))), s0, s1);
+            sw_unpack(sw_fma(sw_mul(dt2, lap), sw_pack(sqrtf(s0), sqrtf(s1)), c), n0, n1);
+            put(z, n0, n1);
+            zb = c;
+            c = zf;
+            if (z + 1 < z1) zf = sw_ld2(p + 2 * PL);
+        }
+    } else {
+        // planes z - 1 (p), z (c), z + 1 (n): row y as L, AB, R, rows y - 1 (m) and y + 1 (q) as AB
+        const float* b = c0p + z0 * PL;
+        float pL = b[-PL - 1], pR = b[-PL + 2], cL = b[-1], cR = b[2], nL = b[PL - 1], nR = b[PL + 2];
+        uint64_t pAB = sw_ld2(b - PL), pm = sw_ld2(b - PL - RS), pq = sw_ld2(b - PL + RS);
+        uint64_t cAB = sw_ld2(b), cm = sw_ld2(b - RS), cq = sw_ld2(b + RS);
+        uint64_t nAB = sw_ld2(b + PL), nm = sw_ld2(b + PL - RS), nq = sw_ld2(b + PL + RS);
+        uint64_t ppAB = 0, nnAB = 0;  // z - 2, z + 2 (25 taps)
+        if (ST == MSBG_BILAPLACIAN) {
+            ppAB = sw_ld2(b - 2 * PL);
+            nnAB = sw_ld2(b + 2 * PL);
+        }
+#pragma unroll 2
+        for (int z = z0; z < z1; ++z) {
+            const float* p = c0p + z * PL;
+            // plane z's diagonal columns: L and R of rows y - 1 and y + 1
+            const float mL = p[-RS - 1], mR = p[-RS + 2], qL = p[RS - 1], qR = p[RS + 2];
+            const uint64_t f0 = cAB, f1 = sw_pack(cL, lo(cAB)), f2 = sw_pack(hi(cAB), cR), f3 = cm, f4 = cq, f5 = pAB, f6 = nAB;
+            const uint64_t fx = sw_mul(sw_sub(f2, f1), half2), fy = sw_mul(sw_sub(f4, f3), half2), fz = sw_mul(sw_sub(f6, f5), half2);
+            // (x+1, y+1), (x+1, y-1), (x-1, y+1), (x-1, y-1) in plane z
+            const uint64_t d1 = sw_pack(hi(cq), qR), d2 = sw_pack(hi(cm), mR), d3 = sw_pack(qL, lo(cq)), d4 = sw_pack(mL, lo(cm));
+            // (x+1, z+1), (x+1, z-1), (x-1, z+1), (x-1, z-1) in row y
+            const uint64_t d5 = sw_pack(hi(nAB), nR), d6 = sw_pack(hi(pAB), pR), d7 = sw_pack(nL, lo(nAB)), d8 = sw_pack(pL, lo(pAB));
+            float n0, n1;
+            if (ST == MSBG_MEAN_CURVATURE) {  // meancurv.rs:50-101
+                const uint64_t q2 = sw_pack(0.25f, 0.25f), m2 = sw_pack(-2.0f, -2.0f), two_f0 = sw_add(f0, f0);
+                const uint64_t fxx = sw_sub(sw_add(f1, f2), two_f0), fyy = sw_sub(sw_add(f3, f4), two_f0), fzz = sw_sub(sw_add(f5, f6), two_f0);
+                const uint64_t fyx = sw_mul(sw_add(sw_sub(sw_sub(d1, d2), d3), d4), q2);
+                const uint64_t fzx = sw_mul(sw_add(sw_sub(sw_sub(d5, d6), d7), d8), q2);
+                const uint64_t fzy = sw_mul(sw_add(sw_sub(sw_sub(nq, pq), nm), pm), q2);
+                const uint64_t i1 = sw_mul(fy, fyx), i2 = sw_mul(fz, fzx), i3 = sw_mul(fz, fzy);
+                const float cr0 = (lo(fx) * lo(i1) + lo(fx) * lo(i2)) + lo(fy) * lo(i3);
+                const float cr1 = (hi(fx) * hi(i1) + hi(fx) * hi(i2)) + hi(fy) * hi(i3);
+                const uint64_t sx = sw_mul(fx, fx), sy = sw_mul(fy, fy), sz = sw_mul(fz, fz);
+                const uint64_t syz = sw_pack(lo(sy) + lo(sz), hi(sy) + hi(sz)), sxz = sw_pack(lo(sx) + lo(sz), hi(sx) + hi(sz)),
+                               sxy = sw_pack(lo(sx) + lo(sy), hi(sx) + hi(sy));
+                const uint64_t hnum = sw_fma(syz, fxx, sw_fma(sxz, fyy, sw_fma(sxy, fzz, sw_mul(m2, sw_pack(cr0, cr1)))));
+                const uint64_t grad = sw_fma(fx, fx, sw_fma(fy, fy, sw_mul(fz, fz)));
+                const float g0 = lo(grad), g1 = hi(grad);
+                const float hc0 = g0 > 1e-7f ? lo(hnum) / g0 : 0.0f, hc1 = g1 > 1e-7f ? hi(hnum) / g1 : 0.0f;
+                float e0, e1;
+                sw_unpack(sw_mul(dt2, sw_pack(hc0, hc1)), e0, e1);
+                sw_unpack(sw_add(f0, sw_pack(clampf(e0, -0.1f, 0.1f), clampf(e1, -0.1f, 0.1f))), n0, n1);
+            } else {  // bilaplacian.rs:45-92
+                const uint64_t g1 = sw_pack(p[-2], cL), g2 = sw_pack(cR, p[3]), g3 = sw_ld2(p - 2 * RS), g4 = sw_ld2(p + 2 * RS);
+                uint64_t s1 = sw_add(f1, f2);
+                s1 = sw_add(s1, f3); s1 = sw_add(s1, f4); s1 = sw_add(s1, f5); s1 = sw_add(s1, f6);
+                uint64_t s2 = sw_add(g1, g2);
+                s2 = sw_add(s2, g3); s2 = sw_add(s2, g4); s2 = sw_add(s2, ppAB); s2 = sw_add(s2, nnAB);
+                uint64_t sd = sw_add(d1, d2);
+                sd = sw_add(sd, d3); sd = sw_add(sd, d4); sd = sw_add(sd, d5); sd = sw_add(sd, d6); sd = sw_add(sd, d7); sd = sw_add(sd, d8);
+                sd = sw_add(sd, nq); sd = sw_add(sd, pq); sd = sw_add(sd, nm); sd = sw_add(sd, pm);
+                const float v0 = 42.0f * lo(f0) - 12.0f * lo(s1), v1 = 42.0f * hi(f0) - 12.0f * hi(s1);
+                const uint64_t hv = sw_add(sw_add(sw_pack(v0, v1), s2), sw_add(sd, sd));  // 2 sd = sd + sd
+                float q0, q1, u0, u1;
+                sw_unpack(sw_fma(fx, fx, sw_fma(fy, fy, sw_mul(fz, fz))), q0, q1);
+                sw_unpack(sw_mul(sw_mul(dt2, hv), sw_pack(sqrtf(q0), sqrtf(q1))), u0, u1);
+                sw_unpack(sw_add(f0, sw_pack(clampf(-u0, -0.1f, 0.1f), clampf(-u1, -0.1f, 0.1f))), n0, n1);
+            }
+            put(z, n0, n1);
+            if (ST == MSBG_BILAPLACIAN) ppAB = pAB;
+            pL = cL; pR = cR; pAB = cAB; pm = cm; pq = cq;
+            cL = nL; cR = nR; cAB = nAB; cm = nm; cq = nq;
+            if (z + 1 < z1) {
+                const float* n = p + 2 * PL;
+                nL = n[-1];
+                nR = n[2];
+                nm = sw_ld2(n - RS);
+                nq = sw_ld2(n + RS);
+                if (ST == MSBG_BILAPLACIAN) {
+                    nAB = nnAB;
+                    nnAB = sw_ld2(n + PL);
+                } else {
+                    nAB = sw_ld2(n);
+                }
+            }
+        }
+    }
+}
+
 // Blocks whose halo leaves the domain at a whole block's face: the Neumann
 // rule (solver.rs:205-209) mirrors halo depth d to the same block layer's cell
 // d - 1 from that face, so such a halo plane is read exactly like an interior
@@ -380,8 +594,18 @@ __device__ __forceinline__ void stage_general(const SweepArgs& a, float* __restr
     stage_general_call<E, BSX, ST, COMPACT, CG>({a.payload, a.coarse, a.bxyz, a.sx, a.sy, a.sz, a.empty, a.full}, h, nb, pi, tab);
 }
 
-template <class E, int BSX, int ST>
-__global__ void __launch_bounds__(BSX * BSX < 32 ? 32 : BSX * BSX, BSX == 16 ? 4 : BSX == 8 ? 12 : 1)
+// Threads of a phase CTA: BSX^2 (8 planes per thread of a 16^3 block) when a
+// phase's blocks fill the chip; phases of fewer blocks are bound by one block's
+// latency, which more threads with fewer planes each shorten (10 sweeps of the
+// 256^3 shell, about 109 blocks a phase, B200: 19 taps u16 0.84 ms with 256
+// threads, 0.39 with 1,024; at about 220 a phase 0.61 with 256, 0.56 with 512,
+// 0.71 with 1,024; at 586 0.48 with 256 and 0.54 with 512).
+template <int BSX> struct PhaseThreads { static constexpr int v = BSX * BSX < 32 ? 32 : BSX * BSX; };
+constexpr int kPhaseWide = 148;    // at most one 16^3 block per SM: 1,024 threads
+constexpr int kPhaseMiddle = 296;  // at most two: 512 threads
+
+template <class E, int BSX, int ST, int NT>
+__global__ void __launch_bounds__(NT, BSX == 16 ? 1024 / NT : BSX == 8 ? 12 : 1)
 sweep_phase_kernel(SweepArgs a, const int32_t* __restrict__ order) {
     constexpr int HALO = ST == MSBG_BILAPLACIAN ? 2 : 1;
     constexpr int HSX = BSX + 2 * HALO;
@@ -416,7 +640,6 @@ sweep_phase_kernel(SweepArgs a, const int32_t* __restrict__ order) {
             // resolution.  Centre and face rows move as
             // 16-byte quads; all loads of a category are issued before its
             // shared-memory stores.
-            constexpr int NT = BSX * BSX < 32 ? 32 : BSX * BSX;
             constexpr int NC4 = N / 4;
             constexpr int KC = (NC4 + NT - 1) / NT;
             const int mir = sides;
@@ -563,7 +786,8 @@ sweep_phase_kernel(SweepArgs a, const int32_t* __restrict__ order) {
             stage_general<E, BSX, ST>(a, h, nb, pi, tab);
         }
         __syncthreads();
-        sweep_compute<E, BSX, ST>(a, h, nb[13], pi, tid);
+        if constexpr (BSX >= 8) sweep_compute_pair<E, BSX, ST, BSX * BSX * BSX / 2 / NT>(a, h, nb[13], pi, tid);
+        else sweep_compute<E, BSX, ST>(a, h, nb[13], pi, tid);
     }
 }
 
@@ -835,41 +1059,6 @@ __device__ __forceinline__ void compute_compact(const SweepArgs& a, const float*
         }
     }
 }
-
-// Pairs of f32 in one 64-bit register and the paired IEEE single-precision
-// operations of sm_100 (each half rounded as the scalar operation).  The
-// stencil below feeds no paired product directly into a paired sum (the
-// code generator may fuse such a pair even with .rn); its products go to
-// explicit fused multiply-adds, as in the scalar form.
-__device__ __forceinline__ uint64_t sw_pack(float a, float b) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void sw_unpack(uint64_t v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t sw_add(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t sw_sub(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t sw_mul(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t sw_fma(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t sw_ld2(const float* p) { return *reinterpret_cast<const uint64_t*>(p); }
 
 // The 7-tap stencil over a block staged in the compact layout, two
 // x-columns per thread: thread (xp, y) walks columns x = 2 xp and x + 1 along
@@ -1487,31 +1676,39 @@ static void wave_items(SweepPlan* plan, msbg_ctx* ctx, int iterations) {
     plan->wave_iters = iterations;
 }
 
-template <class E, int BSX, int ST>
-static void launch_phase(msbg_ctx* ctx, const SweepArgs& a, const int32_t* order, int n) {
+template <class E, int BSX, int ST, int NT>
+static void launch_phase_nt(msbg_ctx* ctx, const SweepArgs& a, const int32_t* order, int n) {
     constexpr int HALO = ST == MSBG_BILAPLACIAN ? 2 : 1;
     constexpr int HSX = BSX + 2 * HALO;
     const size_t smem = sizeof(float) * HSX * HSX * Stage<BSX>::RS;
     static bool attr_set = false;  // per instantiation
     if (!attr_set) {
-        CUDA_CHECK(cudaFuncSetAttribute(sweep_phase_kernel<E, BSX, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CUDA_CHECK(cudaFuncSetAttribute(sweep_phase_kernel<E, BSX, ST, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         // all of the SM's unified L1/shared storage as shared memory: more
         // CTAs (and their staging loads) resident per SM
-        CUDA_CHECK(cudaFuncSetAttribute(sweep_phase_kernel<E, BSX, ST>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        CUDA_CHECK(cudaFuncSetAttribute(sweep_phase_kernel<E, BSX, ST, NT>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                         (int)cudaSharedmemCarveoutMaxShared));
         attr_set = true;
     }
-    const int threads = BSX * BSX < 32 ? 32 : BSX * BSX;
+    begin_launch(ctx);
+    launch_chained(ctx->stream, sweep_phase_kernel<E, BSX, ST, NT>, dim3((unsigned)n), dim3(NT), smem, 1, a, order);
+    after_launch(ctx, "sweep_phase_kernel");
+}
+
+template <class E, int BSX, int ST>
+static void launch_phase(msbg_ctx* ctx, const SweepArgs& a, const int32_t* order, int n) {
     // f32 with one-cell halos: the double-buffered kernel in the compact
     // layout (two 25-tap buffers would leave too few CTAs per SM)
-    if (std::is_same<E, ElemF32>::value && BSX >= 8 && ST != MSBG_BILAPLACIAN) {
+    if constexpr (std::is_same<E, ElemF32>::value && BSX >= 8 && ST != MSBG_BILAPLACIAN) {
         if (a.clamp01) launch_compact<BSX, ST, true>(ctx, a, order, n);
         else launch_compact<BSX, ST, false>(ctx, a, order, n);
-        return;
+    } else {
+        if constexpr (BSX == 16) {
+            if (n <= kPhaseWide) return launch_phase_nt<E, BSX, ST, 1024>(ctx, a, order, n);
+            if (n <= kPhaseMiddle) return launch_phase_nt<E, BSX, ST, 512>(ctx, a, order, n);
+        }
+        launch_phase_nt<E, BSX, ST, PhaseThreads<BSX>::v>(ctx, a, order, n);
     }
-    begin_launch(ctx);
-    launch_chained(ctx->stream, sweep_phase_kernel<E, BSX, ST>, dim3((unsigned)n), dim3((unsigned)threads), smem, 1, a, order);
-    after_launch(ctx, "sweep_phase_kernel");
 }
 
 template <class E, int BSX>
