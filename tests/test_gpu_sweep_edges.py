@@ -62,3 +62,21 @@ def test_multires_edge_blocks_match_oracle(msbg, ctx, oracle, extent, stencil):
     ctx.synchronize()
     oracle.sweep_multires(fine, coarse, levels, active, stencil, 0.05, 3, False)
     assert_same_blocks(dfine, fine, active)
+
+
+@pytest.mark.parametrize("iterations", [1, 2, 11])
+@pytest.mark.parametrize("stencil", [0, 1])
+@pytest.mark.parametrize("extent,keep", [((64, 64, 64), 0.7), ((256, 256, 192), 0.02)])
+def test_active_lists_in_any_order(msbg, ctx, oracle, extent, keep, stencil, iterations):
+    """Active lists with repeats, absent and constant blocks, in no order, on
+    grids that are mostly active (codes from an array) and mostly empty (codes
+    from the block map); one, few and many sweeps in a launch."""
+    sx, sy, sz = extent
+    host = random_sparse(msbg, sx, sy, sz, 8, keep, 5 + stencil, empty=0.1, full=0.9)
+    r = np.random.default_rng(sx + iterations)
+    active = list(host.blocks) + list(host.full)[:20] + list(r.integers(0, host.n_blocks, 30)) + list(host.blocks)[::3]
+    r.shuffle(active)
+    active = [int(b) for b in active]
+    dev = run_device(msbg, ctx, host, active, stencil, 0.05, iterations, False)
+    oracle.sweep(host, active, stencil, 0.05, iterations, False)
+    assert_same_blocks(dev, host, np.arange(host.n_blocks))
