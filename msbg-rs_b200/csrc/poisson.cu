@@ -2246,6 +2246,58 @@ struct msbg_batch {
 
 namespace msbg {
 
+// Captures each group's cycle as a branch of its own, so that the groups run
+// side by side: they share no buffer, and their many small launches leave
+// most of the chip idle (16 problems in two groups, B200: 7.26 -> 5.30 ms a
+// solve).  Group 0 stays on the context's stream; the others take streams
+// that live until the capture has ended.
+struct GroupFork {
+    msbg_ctx* ctx;
+    cudaStream_t home;
+    std::vector<cudaStream_t> side;
+    std::vector<cudaEvent_t> ends;
+    cudaEvent_t begin = nullptr;
+    GroupFork(msbg_ctx* c, int ng) : ctx(c), home(c->stream) {
+        try {
+            int priority = 0;
+            CUDA_CHECK(cudaStreamGetPriority(home, &priority));
+            CUDA_CHECK(cudaEventCreateWithFlags(&begin, cudaEventDisableTiming));
+            for (int g = 1; g < ng; ++g) {
+                cudaStream_t s = nullptr;
+                CUDA_CHECK(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, priority));
+                side.push_back(s);
+                cudaEvent_t e = nullptr;
+                CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+                ends.push_back(e);
+            }
+        } catch (...) {
+            release();
+            throw;
+        }
+    }
+    GroupFork(const GroupFork&) = delete;
+    GroupFork& operator=(const GroupFork&) = delete;
+    ~GroupFork() { release(); }
+    void open() {
+        CUDA_CHECK(cudaEventRecord(begin, home));
+        for (cudaStream_t s : side) CUDA_CHECK(cudaStreamWaitEvent(s, begin, 0));
+    }
+    void enter(int g) { ctx->stream = g ? side[g - 1] : home; }
+    void join() {
+        enter(0);
+        for (size_t i = 0; i < side.size(); ++i) {
+            CUDA_CHECK(cudaEventRecord(ends[i], side[i]));
+            CUDA_CHECK(cudaStreamWaitEvent(home, ends[i], 0));
+        }
+    }
+    void release() {
+        enter(0);
+        for (cudaEvent_t e : ends) cudaEventDestroy(e);
+        for (cudaStream_t s : side) cudaStreamDestroy(s);
+        if (begin) cudaEventDestroy(begin);
+    }
+};
+
 static void batch_group_build(msbg_poisson* P, int bsx, const std::vector<int>& probs, const uint64_t* dims,
                               const uint64_t* const* active, const size_t* n_active) {
     int64_t NX = 1, NY = 1, nzmax = 1;
@@ -2692,6 +2744,7 @@ int msbg_batch_solve(msbg_batch* B, double tol, int iters_per_cycle, int max_cyc
         CUDA_CHECK(cudaGraphCreate(&G, 0));
         const uint64_t l0 = ctx->launches;
         bool capturing = false;
+        GroupFork fork(ctx, ng);  // its streams outlive the capture
         try {
             cudaGraphConditionalHandle h;
             CUDA_CHECK(cudaGraphConditionalHandleCreate(&h, G, 0, 0));
@@ -2716,8 +2769,12 @@ int msbg_batch_solve(msbg_batch* B, double tol, int iters_per_cycle, int max_cyc
             // its body: one cycle of every group, then the test
             CUDA_CHECK(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
             capturing = true;
-            for (int g = 0; g < ng; ++g)
+            fork.open();
+            for (int g = 0; g < ng; ++g) {
+                fork.enter(g);
                 batch_cycle(B->groups[g], B->x[g].as<double>(), B->b[g].as<float>(), iters_per_cycle, tol);
+            }
+            fork.join();
             begin_launch(ctx);
             bk_loop_ctrl<<<1, 256, 0, ctx->stream>>>(h, gt, ng, ctrl, 1);
             after_launch(ctx, "bk_loop_ctrl");
@@ -2725,6 +2782,7 @@ int msbg_batch_solve(msbg_batch* B, double tol, int iters_per_cycle, int max_cyc
             capturing = false;
             CUDA_CHECK(cudaGraphInstantiate(&B->exec, G, 0));
         } catch (...) {
+            fork.enter(0);
             if (capturing) {
                 cudaGraph_t tmp = nullptr;
                 cudaStreamEndCapture(ctx->stream, &tmp);
