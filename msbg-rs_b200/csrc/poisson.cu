@@ -1989,9 +1989,31 @@ __global__ void __launch_bounds__(256) bk_block_dot(int64_t nblocks, int cells, 
     }
 }
 
-// scal[p][slot] = sum of the partials of problem p's blocks (one warp per problem)
+// What a problem's scalars become once a sum has arrived.  SEG_ALPHA: alpha =
+// rz / pq; SEG_BETA: beta = rz_new / rz, rz = rz_new, one more iteration
+// counted; SEG_TEST: active = (r.r > tol^2 b.b).  Problems that are not active
+// get alpha = beta = 0 and stay where they are.
+enum { SEG_NONE = 0, SEG_ALPHA, SEG_BETA, SEG_TEST };
+
+__device__ __forceinline__ void seg_scalars(double* S, int op, double tol2) {
+    const bool on = S[S_ACTIVE] > 0.0;
+    if (op == SEG_ALPHA) {
+        S[S_ALPHA] = (on && S[S_PQ] > 0.0) ? S[S_RZ] / S[S_PQ] : 0.0;
+    } else if (op == SEG_BETA) {
+        S[S_BETA] = (on && S[S_RZ] > 0.0) ? S[S_RZN] / S[S_RZ] : 0.0;
+        S[S_RZ] = S[S_RZN];
+        if (on) S[S_ITER] += 1.0;
+    } else if (op == SEG_TEST) {
+        S[S_ACTIVE] = S[S_RR] > tol2 * S[S_BB] ? 1.0 : 0.0;
+    }
+}
+
+// scal[p][slot] = sum of the partials of problem p's blocks (one warp per
+// problem), then the scalars that follow from it.  Launches bound these
+// kernels: with the scalars here and both updates in bk_update, three fewer per
+// iteration, the solve of 16 problems takes 5.24 instead of 5.30 ms (B200).
 __global__ void bk_seg_sum(int np, const int64_t* __restrict__ pb, const double* part, double* __restrict__ scal,
-                           int slot) {
+                           int slot, int op, double tol2) {
     chain_trigger();
     chain_wait();
     const int lane = threadIdx.x & 31;
@@ -2001,38 +2023,12 @@ __global__ void bk_seg_sum(int np, const int64_t* __restrict__ pb, const double*
         for (int64_t k = pb[p] + lane; k < pb[p + 1]; k += 32) s += part[k];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) scal[(int64_t)p * S_WIDTH + slot] = s;
-    }
-}
-
-// op 0: alpha = rz / pq; op 1: beta = rz_new / rz, rz = rz_new, one more
-// iteration counted; op 2: active = (r.r > tol^2 b.b).  Problems that are not
-// active get alpha = beta = 0 and stay where they are.
-__global__ void bk_scalars(int np, double* __restrict__ scal, int op, double tol2) {
-    chain_trigger();
-    chain_wait();
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
-        double* S = scal + (int64_t)p * S_WIDTH;
-        const bool on = S[S_ACTIVE] > 0.0;
-        if (op == 0) {
-            S[S_ALPHA] = (on && S[S_PQ] > 0.0) ? S[S_RZ] / S[S_PQ] : 0.0;
-        } else if (op == 1) {
-            S[S_BETA] = (on && S[S_RZ] > 0.0) ? S[S_RZN] / S[S_RZ] : 0.0;
-            S[S_RZ] = S[S_RZN];
-            if (on) S[S_ITER] += 1.0;
-        } else {
-            S[S_ACTIVE] = S[S_RR] > tol2 * S[S_BB] ? 1.0 : 0.0;
+        if (lane == 0) {
+            double* S = scal + (int64_t)p * S_WIDTH;
+            S[slot] = s;
+            seg_scalars(S, op, tol2);
         }
     }
-}
-
-// y += sign * s_p x  (s_p = scal[problem of the cell's block][slot])
-__global__ void bk_axpy(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* scal, int slot,
-                        float sign, const float* x, float* __restrict__ y) {
-    chain_trigger();
-    chain_wait();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        y[i] += (float)(sign * scal[(int64_t)blk_prob[i >> lg3] * S_WIDTH + slot]) * x[i];
 }
 
 // p = z + beta_p p
@@ -2044,31 +2040,29 @@ __global__ void bk_xpay(int64_t n, int lg3, const int32_t* __restrict__ blk_prob
         p[i] = z[i] + (float)scal[(int64_t)blk_prob[i >> lg3] * S_WIDTH + S_BETA] * p[i];
 }
 
-// x64 += alpha_p p
-__global__ void bk_add64(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* scal,
-                         const float* p, double* __restrict__ x) {
+// x64 += alpha_p p, r -= alpha_p q
+__global__ void bk_update(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* scal,
+                          const float* p, const float* q, double* __restrict__ x, float* __restrict__ r) {
     chain_trigger();
     chain_wait();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        x[i] += scal[(int64_t)blk_prob[i >> lg3] * S_WIDTH + S_ALPHA] * (double)p[i];
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double alpha = scal[(int64_t)blk_prob[i >> lg3] * S_WIDTH + S_ALPHA];
+        x[i] += alpha * (double)p[i];
+        r[i] += (float)(-1.0f * alpha) * q[i];
+    }
 }
 
-static void seg_dot(msbg_poisson* P, const float* a, const float* b, int slot) {
+static void seg_dot(msbg_poisson* P, const float* a, const float* b, int slot, int op = SEG_NONE, double tol = 0.0) {
     const PLevelDev& F = P->lv[0];
     const int cells = F.bs * F.bs * F.bs;
     begin_launch(P->ctx);
     launch_chained(P->ctx->stream, bk_block_dot, (unsigned)std::min<int64_t>(F.n(), 148 * 8), 256, 0, 1, F.n(), cells, a, b,
-                                                                                         P->bpart.as<double>());
+                   P->bpart.as<double>());
     after_launch(P->ctx, "bk_block_dot");
     begin_launch(P->ctx);
-    launch_chained(P->ctx->stream, bk_seg_sum, (unsigned)((P->np * 32 + 255) / 256), 256, 0, 1, P->np, P->d_prob_blocks.as<int64_t>(), P->bpart.as<double>(), P->scal.as<double>(), slot);
+    launch_chained(P->ctx->stream, bk_seg_sum, (unsigned)((P->np * 32 + 255) / 256), 256, 0, 1, P->np,
+                   P->d_prob_blocks.as<int64_t>(), P->bpart.as<double>(), P->scal.as<double>(), slot, op, tol * tol);
     after_launch(P->ctx, "bk_seg_sum");
-}
-
-static void scalars(msbg_poisson* P, int op, double tol) {
-    begin_launch(P->ctx);
-    launch_chained(P->ctx->stream, bk_scalars, (unsigned)((P->np + 127) / 128), 128, 0, 1, P->np, P->scal.as<double>(), op, tol * tol);
-    after_launch(P->ctx, "bk_scalars");
 }
 
 // Start of a batched solve (not captured): r = b - A x, b.b, r.r, active flags.
@@ -2078,8 +2072,7 @@ static void batch_start(msbg_poisson* P, double* x64, const float* b, double tol
     CUDA_CHECK(cudaMemsetAsync(P->scal.p, 0, (size_t)P->np * S_WIDTH * 8, P->ctx->stream));
     launch_residual64(P, x64, b, r);
     seg_dot(P, b, b, S_BB);
-    seg_dot(P, r, r, S_RR);
-    scalars(P, 2, tol);
+    seg_dot(P, r, r, S_RR, SEG_TEST, tol);
     (void)n;
 }
 
@@ -2103,24 +2096,18 @@ static void batch_cycle(msbg_poisson* P, double* x64, const float* b, int K, dou
     seg_dot(P, r, z, S_RZ);
     for (int k = 0; k < K; ++k) {
         launch_matvec(P, 0, p, q);
-        seg_dot(P, p, q, S_PQ);
-        scalars(P, 0, tol);
+        seg_dot(P, p, q, S_PQ, SEG_ALPHA);
         begin_launch(ctx);
-        launch_chained(ctx->stream, bk_add64, grid_for(n), 256, 0, 1, n, lg3, bp, sc, p, x64);
-        after_launch(ctx, "bk_add64");
-        begin_launch(ctx);
-        launch_chained(ctx->stream, bk_axpy, grid_for(n), 256, 0, 1, n, lg3, bp, sc, S_ALPHA, -1.0f, q, r);
-        after_launch(ctx, "bk_axpy");
+        launch_chained(ctx->stream, bk_update, grid_for(n), 256, 0, 1, n, lg3, bp, sc, p, q, x64, r);
+        after_launch(ctx, "bk_update");
         vcycle(P, 0, z, r, true);
-        seg_dot(P, r, z, S_RZN);
-        scalars(P, 1, tol);
+        seg_dot(P, r, z, S_RZN, SEG_BETA);
         begin_launch(ctx);
         launch_chained(ctx->stream, bk_xpay, grid_for(n), 256, 0, 1, n, lg3, bp, sc, z, p);
         after_launch(ctx, "bk_xpay");
     }
     launch_residual64(P, x64, b, r);
-    seg_dot(P, r, r, S_RR);
-    scalars(P, 2, tol);
+    seg_dot(P, r, r, S_RR, SEG_TEST, tol);
 }
 
 // Autotuner: for every level but the coarsest, time each choice on the
