@@ -538,7 +538,7 @@ int msbg_unet_train_step_device(msbg_unet* net, const float* d_r, const float* d
  * its group's vectors (msbg_batch_problem), blocks in ascending id order.
  * msbg_batch_buffers gives the group's device right-hand side (f32) and
  * solution (FP64).  tune != 0 autotunes every level but the coarsest: the
- * z-planes per CTA (2, 4, 8 or 16) of the 16^3 tile kernel on levels of whole
+ * z-planes per CTA (2, 4, 8 or 16) of the 16^3 tile kernels on levels of whole
  * 16^3 blocks, the launch shapes (threads, CTAs per SM) of the Jacobi and
  * residual kernels elsewhere (msbg_batch_tuning: per level cfg_out[3l..3l+2]
  * = Jacobi shape index, residual shape index, tile z-planes or 0, and the
