@@ -547,15 +547,21 @@ struct TransferArgs {
     int64_t cells;          // cells of the level the kernel runs over
 };
 
+// Four lanes form a coarse cell: lane tz the four x-sums of its fine plane, which
+// lane 0 then adds plane by plane.  The levels this runs on are small (a few
+// thousand cells), so it is bound by one thread's chain of address arithmetic
+// and loads: 16 of them instead of 64 (B200, solve of 3.18 M cells 2.56 -> 2.42
+// ms, 16 batched solves 4.88 -> 4.71).
 __global__ void pk_restrict(TransferArgs T, const float* r, float* __restrict__ bc) {
     chain_trigger();
-    chain_wait();
     const int bsc = 1 << T.lgc, mc = bsc - 1, mf = (1 << T.lgf) - 1;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T.cells; i += (int64_t)gridDim.x * blockDim.x) {
-        if (T.diag && !(T.diag[i] > 0.0f)) {
-            bc[i] = 0.0f;
-            continue;
-        }
+    const int tz = threadIdx.x & 3;
+    bool waited = false;
+    // a warp's lanes take the same rounds; cells past the end repeat the last one
+    for (int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31)) >> 2; i0 < T.cells;
+         i0 += ((int64_t)gridDim.x * blockDim.x) >> 2) {
+        const int64_t iw = i0 + ((threadIdx.x & 31) >> 2), i = min(iw, T.cells - 1);
+        const bool on = !T.diag || T.diag[i] > 0.0f;
         const int64_t k = i >> (3 * T.lgc);
         const int v = (int)(i & ((1 << (3 * T.lgc)) - 1));
         const int q[3] = {T.coords[3 * k] * bsc + (v & mc), T.coords[3 * k + 1] * bsc + ((v >> T.lgc) & mc),
@@ -565,28 +571,31 @@ __global__ void pk_restrict(TransferArgs T, const float* r, float* __restrict__ 
         for (int a = 0; a < 3; ++a) fb0[a] = ((2 * T.coords[3 * k + a] * bsc) >> T.lgf) - 1;
         const int32_t* nb = T.nb + k * 64;
         const float w1[4] = {0.25f, 0.75f, 0.75f, 0.25f};
+        const int gz = 2 * q[2] - 1 + tz, bz = (gz >> T.lgf) - fb0[2];
+        int64_t at[16];  // of the lane's 16 fine cells, -1: absent
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            const int gy = 2 * q[1] - 1 + e / 4, by = (gy >> T.lgf) - fb0[1], gx = 2 * q[0] - 1 + e % 4, bx = (gx >> T.lgf) - fb0[0];
+            const int32_t sl = nb[bx + 4 * by + 16 * bz];
+            at[e] = sl >= 0 && on ? ((int64_t)sl << (3 * T.lgf)) + ((gx & mf) | ((gy & mf) << T.lgf) | ((gz & mf) << (2 * T.lgf))) : -1;
+        }
+        if (!waited) chain_wait();  // the tables belong to no kernel in flight
+        waited = true;
+        float row[4];
+#pragma unroll
+        for (int ty = 0; ty < 4; ++ty) {
+            row[ty] = 0.0f;
+#pragma unroll
+            for (int tx = 0; tx < 4; ++tx) row[ty] += w1[tx] * (at[4 * ty + tx] >= 0 ? r[at[4 * ty + tx]] : 0.0f);
+        }
         float s = 0.0f;
 #pragma unroll
-        for (int tz = 0; tz < 4; ++tz) {
-            const int gz = 2 * q[2] - 1 + tz, bz = (gz >> T.lgf) - fb0[2];
+        for (int z = 0; z < 4; ++z)
 #pragma unroll
-            for (int ty = 0; ty < 4; ++ty) {
-                const int gy = 2 * q[1] - 1 + ty, by = (gy >> T.lgf) - fb0[1];
-                float row = 0.0f;
-#pragma unroll
-                for (int tx = 0; tx < 4; ++tx) {
-                    const int gx = 2 * q[0] - 1 + tx, bx = (gx >> T.lgf) - fb0[0];
-                    const int32_t sl = nb[bx + 4 * by + 16 * bz];
-                    const float val = sl >= 0 ? r[((int64_t)sl << (3 * T.lgf)) + ((gx & mf) | ((gy & mf) << T.lgf) |
-                                                                                   ((gz & mf) << (2 * T.lgf)))]
-                                              : 0.0f;
-                    row += w1[tx] * val;
-                }
-                s += (w1[ty] * w1[tz]) * row;
-            }
-        }
-        bc[i] = s * 0.125f;
+            for (int ty = 0; ty < 4; ++ty) s += (w1[ty] * w1[z]) * __shfl_sync(0xffffffffu, row[ty], z, 4);
+        if (tz == 0 && iw < T.cells) bc[i] = on ? s * 0.125f : 0.0f;
     }
+    if (!waited) chain_wait();
 }
 
 // x_f += P x_c at the active fine cells.
@@ -1237,7 +1246,7 @@ static void vcycle(msbg_poisson* P, int l, float* x, const float* b, bool x_zero
         else launch_chained(P->ctx->stream, pk_restrict_tile<2, 64>, nb, 64, 0, 1, R, F.r.as<float>(), C.b.as<float>());
         after_launch(P->ctx, "pk_restrict_tile");
     } else {
-        launch_chained(P->ctx->stream, pk_restrict, grid_for(C.cells()), 256, 0, 1, R, F.r.as<float>(), C.b.as<float>());
+        launch_chained(P->ctx->stream, pk_restrict, grid_for(4 * C.cells()), 256, 0, 1, R, F.r.as<float>(), C.b.as<float>());
         after_launch(P->ctx, "pk_restrict");
     }
     vcycle(P, l + 1, C.x.as<float>(), C.b.as<float>(), true);
