@@ -491,7 +491,7 @@ def algorithmic_bytes(kernel, n, n_fine, n_active, launches):
     """Algorithmic HBM bytes moved by `launches` launches of `kernel` in one
     FLIP transfer step's accounting: 8 B per f32 cell-update for the in-place
     smoother; 28 B per particle once per P2G for the splat (position, velocity
-    and mass read once: P2G_SPLAT_LAUNCHES launches make one P2G); 24 B
+    and mass read once: one launch makes one P2G); 24 B
     written per face-cell of the active blocks for the combine; 12 B read + 12
     B written per particle for G2P; 24 B per element per onesweep radix pass
     (3 passes per sort)."""
@@ -499,9 +499,7 @@ def algorithmic_bytes(kernel, n, n_fine, n_active, launches):
         return 8.0 * n_fine * 4096 * SWEEPS * launches
     if kernel in SWEEP_KERNELS:
         return 8.0 * n_fine * 4096 * SWEEPS * launches / 80
-    if kernel == "p2g_cells_kernel":
-        return 28.0 * n * launches / P2G_SPLAT_LAUNCHES
-    if kernel == "p2g_r2_kernel":
+    if kernel in ("p2g_cells_kernel", "p2g_r2_kernel"):
         return 28.0 * n * launches
     if kernel == "p2g_combine_kernel":
         return 24.0 * n_active * 4096 * launches
@@ -514,25 +512,17 @@ def algorithmic_bytes(kernel, n, n_fine, n_active, launches):
     return None
 
 
-# Launches of the general splat kernel per P2G (one per face direction; the
-# r_p = 2 kernel does the three directions in one launch).
-P2G_SPLAT_LAUNCHES = 3
-
 # DRAM bytes (read + write) per launch measured by ncu on a smaller case of
-# the same kernel, per unit of work: p2g_cells_kernel at 128^3 (5,767,168
-# particles, one direction per launch) read 167.28 MB and wrote 3.96 MB
-# (profiles/p2g_cells_kernel_flip128.txt); traffic grows with the particle
-# count, so it is scaled by particles.
-TRAFFIC_PER_UNIT = {"p2g_cells_kernel": (167.28e6 + 3.96e6) / 5767168,
-                    # r_p = 2 kernel, all three directions in one launch at 128^3
-                    # (profiles/p2g_r2_kernel_flip128.txt): 308.83 MB read, 47.21 MB written
-                    "p2g_r2_kernel": (308.83e6 + 47.21e6) / 5767168}
+# the same kernel, per unit of work: p2g_r2_kernel, all three directions in one
+# launch, at 128^3 (5,767,168 particles, profiles/p2g_r2_kernel_flip128.txt)
+# read 308.83 MB and wrote 47.21 MB; traffic grows with the particle count, so it is
+# scaled by particles.
+TRAFFIC_PER_UNIT = {"p2g_r2_kernel": (308.83e6 + 47.21e6) / 5767168}
 
-# Warp instructions per unit of work from the same capture (575,950,823 per
-# launch at 128^3): the splat is bound by instruction issue, not by DRAM, so
-# its second roofline is issue slots (4 warp instructions per SM per clock).
-INST_PER_UNIT = {"p2g_cells_kernel": 575950823 / 5767168,
-                 "p2g_r2_kernel": 1073931570 / 5767168}
+# Warp instructions per unit of work from the same capture: the splat is bound
+# by instruction issue, not by DRAM, so its second roofline is issue slots (4
+# warp instructions per SM per clock).
+INST_PER_UNIT = {"p2g_r2_kernel": 1073931570 / 5767168}
 
 
 # The smoother's sweep kernels (one of them runs, by element type, halo and
