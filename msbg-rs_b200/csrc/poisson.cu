@@ -2788,11 +2788,11 @@ int msbg_batch_solve(msbg_batch* B, double tol, int iters_per_cycle, int max_cyc
         }
         const GroupScal* gt = B->gtab.as<GroupScal>();
         long long* ctrl = B->ctrl.as<long long>();
+        GroupFork fork(ctx, ng);  // its streams outlive the capture
         cudaGraph_t G = nullptr;
         CUDA_CHECK(cudaGraphCreate(&G, 0));
         const uint64_t l0 = ctx->launches;
         bool capturing = false;
-        GroupFork fork(ctx, ng);  // its streams outlive the capture
         try {
             cudaGraphConditionalHandle h;
             CUDA_CHECK(cudaGraphConditionalHandleCreate(&h, G, 0, 0));
