@@ -569,8 +569,10 @@ __device__ __forceinline__ void splat_cells_body(const SplatArgs& a, const int k
                 }
             }
             if (odd) {
-                // rows beyond the compact ones, particle by particle
+                // rows beyond the compact ones, particle by particle: they fall
+                // on window words that other lanes have just added to
                 if (deps_pending) wait_deps();
+                __syncwarp();
 #pragma unroll 1
                 for (int j = s0; j < s1; ++j) {
                     const float4 P = wslot[j - s0], R = wslot[CAP + j - s0];

@@ -1,0 +1,48 @@
+"""P2G of particles on cell faces (integer coordinates): with r_p - 1/2 an
+integer their footprints have one row more per lane axis than the splat's cell
+groups take together, and those rows fall on window words that the groups of
+neighbouring cells add to.  Whole lattices and lattices mixed with free
+particles, in tiles of one staged chunk and of several: every face within one
+ulp of the FP64 sum of the reference's f32 terms, and the same bits each time."""
+import numpy as np
+import pytest
+
+from test_gpu_particles import device_channels, ulp_diff
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bsx", [8, 16])
+@pytest.mark.parametrize("r_p", [1.5, 2.5])
+@pytest.mark.parametrize("copies,free", [(1, 0), (3, 20000), (20, 5000)])
+def test_particles_on_cell_faces(msbg, ctx, oracle, r_p, bsx, copies, free):
+    r = np.random.default_rng(copies + bsx)
+    f = np.float32
+    axis = np.arange(1, 31, dtype=f)
+    lattice = np.stack(np.meshgrid(axis, axis, axis, indexing="ij"), -1).reshape(-1, 3)
+    if copies > 3:
+        lattice = lattice[np.all((lattice > 6) & (lattice < 19), axis=1)]
+    lattice = np.repeat(lattice, copies, axis=0)
+    # on all three axes, on two and on one
+    off = r.integers(0, 3, len(lattice))
+    lattice[off == 1, 0] += f(0.375)
+    lattice[off == 2, 1:] += f([0.25, 0.8125])
+    pos = np.concatenate([lattice, r.uniform(0, 31.99, (free, 3)).astype(f)]).astype(f)
+    pos = pos[r.permutation(len(pos))]
+    vel = r.normal(size=pos.shape).astype(f)
+    mass = r.uniform(0.5, 1.5, len(pos)).astype(f)
+    want_act = oracle.active_blocks(pos, 32, 32, 32, bsx, r_p)
+    terms = oracle.p2g_terms_f64(pos, vel, mass, 32, 32, 32, bsx, r_p, want_act)
+    first = None
+    for _ in range(3):
+        mac = msbg.MacGrid(ctx, 32, 32, 32, bsx)
+        msbg.particles_to_grid(mac, pos, vel, mass, r_p)
+        act = mac.active_blocks()
+        assert np.array_equal(act.astype(np.int64), want_act)
+        got = device_channels(mac, act)
+        for a in range(3):
+            assert ulp_diff(got[a], terms[a].astype(f)).max() <= 1.0
+        if first is None:
+            first = got
+        for a in range(6):
+            assert np.array_equal(got[a], first[a])
