@@ -2047,11 +2047,14 @@ static void sweep(msbg_grid* g, msbg_grid* coarse, const uint8_t* levels, const 
         if (stream_pos && g->dtype == MSBG_U8) *stream_pos = pos0 + (uint64_t)iterations * chunks_per_sweep;
         return;
     }
+    // (every buffer that a launch bakes in is in the key: the item list moves
+    // when a call of more sweeps outgrows it)
+    const void* items = wave ? plan->wave_items.p : nullptr;
     uint64_t key = 0xcbf29ce484222325ULL;
     auto bits = [](float f) { uint32_t u; memcpy(&u, &f, 4); return (uint64_t)u; };
     for (uint64_t v : {(uint64_t)iterations, (uint64_t)stencil, bits(dt), (uint64_t)a.clamp01, (uint64_t)(uintptr_t)a.payload,
-                       (uint64_t)(uintptr_t)a.coarse, (uint64_t)(uintptr_t)a.xface, (uint64_t)(uintptr_t)prog, bits(a.empty),
-                       bits(a.full)})
+                       (uint64_t)(uintptr_t)a.coarse, (uint64_t)(uintptr_t)a.xface, (uint64_t)(uintptr_t)prog,
+                       (uint64_t)(uintptr_t)items, bits(a.empty), bits(a.full)})
         key = fnv(key, v);
     SweepPlan::Graph* sg = nullptr;
     for (auto& q : plan->graphs)
