@@ -11,6 +11,8 @@
 // constant values.  A host mirror of the table drives materialisation.
 #pragma once
 
+#include <atomic>
+
 #include "common.cuh"
 
 namespace msbg {
@@ -56,6 +58,12 @@ struct HostHash {
 
 struct SweepPlan;
 
+// A number no other grid of the process has had or will have.
+inline uint64_t next_grid_id() {
+    static std::atomic<uint64_t> last{0};
+    return ++last;
+}
+
 }  // namespace msbg
 
 struct msbg_grid {
@@ -69,6 +77,9 @@ struct msbg_grid {
     std::unordered_map<uint64_t, int32_t> map;  // bid -> slot or kCodeFull
     std::vector<uint64_t> slot_bid;             // slot -> bid
     uint64_t version = 0;                       // bumps when the block set changes
+    // What a cached plan remembers this grid by (with `version`): an address can
+    // come back with another grid behind it.
+    const uint64_t id = msbg::next_grid_id();
 
     // device state
     msbg::DevBuf payload;

@@ -1795,7 +1795,7 @@ static SweepPlan* get_plan(msbg_grid* g, msbg_grid* coarse, const uint8_t* level
     uint64_t key = 0xcbf29ce484222325ULL;
     key = fnv(key, n);
     key = fnv(key, g->version);
-    key = fnv(key, (uint64_t)(uintptr_t)coarse);
+    key = fnv(key, coarse ? coarse->id : 0);
     if (coarse) {
         key = fnv(key, coarse->version);
         key = fnv(key, coarse->n_slots());
