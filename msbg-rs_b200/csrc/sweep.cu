@@ -1652,31 +1652,59 @@ static void wave_items(SweepPlan* plan, msbg_ctx* ctx, int iterations) {
     const size_t n = plan->n;
     MSBG_REQUIRE(n < (1u << 24), "too many blocks for a one-launch sweep");
     MSBG_REQUIRE(iterations < (1 << 20), "too many sweeps for a one-launch sweep");
-    // wavefront K holds the blocks of colour c at layer bz of sweep t with
+    // Wavefront K holds the blocks of colour c at layer bz of sweep t with
     // 8 t + c + bz = K.  Within it the higher block layer goes first (a
     // dependency one layer up can tie with its dependant; one at the same
-    // layer or below never does), that is the lower 8 t + c, then the plan
-    // index: the lists of every (colour, layer), joined in that order.
-    int32_t layers = 0;
+    // layer or below never does), then the plan index.
+    // Host time counts: it follows the active blocks and not the domain's
+    // height, which may be millions of layers.
+    std::vector<uint32_t> list(n), next(n);  // plan indices by layer (11 bits at a time), inside one in plan order
     for (size_t i = 0; i < n; ++i) {
         MSBG_REQUIRE((uint64_t)plan->h_bz[i] < (1u << 21), "block layer out of range");
-        layers = std::max(layers, plan->h_bz[i] + 1);
+        list[i] = (uint32_t)i;
     }
-    std::vector<uint32_t> start((size_t)layers * 8 + 1, 0), list(n);
-    for (size_t i = 0; i < n; ++i) ++start[(size_t)plan->h_col[i] * layers + plan->h_bz[i] + 1];
-    for (size_t b = 1; b < start.size(); ++b) start[b] += start[b - 1];
-    {
-        std::vector<uint32_t> at(start.begin(), start.end() - 1);
-        for (size_t i = 0; i < n; ++i) list[at[(size_t)plan->h_col[i] * layers + plan->h_bz[i]]++] = (uint32_t)i;
+    for (int shift = 0; shift < 22; shift += 11) {
+        uint32_t at[2049] = {0};
+        for (size_t i = 0; i < n; ++i) ++at[((plan->h_bz[i] >> shift) & 2047) + 1];
+        for (int d = 0; d < 2048; ++d) at[d + 1] += at[d];
+        for (uint32_t i : list) next[at[(plan->h_bz[i] >> shift) & 2047]++] = i;
+        list.swap(next);
+    }
+    // The runs of one layer and colour (plan indices are colour-major).  A run
+    // is in the wavefronts s, s + 8, ... of its sweeps, s = c + bz; in each
+    // residue class of s the runs, by layer, are by s as well.
+    struct Run {
+        int64_t s;
+        size_t begin, end;
+    };
+    std::vector<Run> runs[8];
+    for (size_t b = 0, e; b < n; b = e) {
+        const int32_t bz = plan->h_bz[list[b]], c = plan->h_col[list[b]];
+        for (e = b + 1; e < n && plan->h_bz[list[e]] == bz && plan->h_col[list[e]] == c;) ++e;
+        runs[(c + bz) & 7].push_back({(int64_t)c + bz, b, e});
     }
     std::vector<int2> items;
     items.reserve(n * (size_t)iterations);
-    const int64_t steps = 8 * (int64_t)iterations;
-    for (int64_t K = 0; K < steps + layers - 1; ++K)
-        for (int64_t q = std::max<int64_t>(0, K - layers + 1); q <= std::min(K, steps - 1); ++q) {
-            const size_t b = (size_t)(q & 7) * layers + (size_t)(K - q);
-            for (uint32_t e = start[b]; e < start[b + 1]; ++e) items.push_back(make_int2((int)(q >> 3), (int)list[e]));
+    size_t lo[8] = {0}, hi[8] = {0};  // the runs of a class that are in its present wavefront
+    int idle = 0;                     // wavefronts in a row without a run
+    for (int64_t K = 0; items.size() < n * (size_t)iterations; ++K) {
+        const int q = (int)(K & 7);
+        const std::vector<Run>& r = runs[q];
+        while (hi[q] < r.size() && r[hi[q]].s <= K) ++hi[q];
+        while (lo[q] < hi[q] && r[lo[q]].s + 8 * (int64_t)(iterations - 1) < K) ++lo[q];
+        for (size_t u = hi[q]; u-- > lo[q];) {
+            const Run run = r[u];
+            const int t = (int)((K - run.s) >> 3);
+            for (size_t e = run.begin; e < run.end; ++e) items.push_back(make_int2(t, (int)list[e]));
         }
+        idle = lo[q] < hi[q] ? 0 : idle + 1;
+        if (idle < 8) continue;
+        int64_t s = INT64_MAX;  // nothing before the next run begins
+        for (int p = 0; p < 8; ++p)
+            if (hi[p] < runs[p].size()) s = std::min(s, runs[p][hi[p]].s);
+        if (s < INT64_MAX) K = s - 1;
+        idle = 0;
+    }
     plan->wave_items.reserve(items.size() * sizeof(int2));
     CUDA_CHECK(cudaMemcpyAsync(plan->wave_items.p, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice,
                                ctx->stream));

@@ -1,6 +1,8 @@
 """Sweep calls that follow one another on one grid: what a call keeps for the
 next (plan, item list, captured launches) has to fit the next call's own sweep
 count, active set and levels.  Bit for bit against the oracle."""
+import time
+
 import numpy as np
 import pytest
 
@@ -54,3 +56,38 @@ def test_coarse_level_made_anew(msbg, ctx, oracle):
         oracle.sweep_multires(fine, coarse, levels, active, 1, 0.05, 1, False)
         assert_same_blocks(dfine, fine, active)
         dcoarse.close()
+
+
+def test_few_blocks_of_a_tall_domain(msbg, ctx):
+    """Blocks near the top of a domain of 2^20 block layers: the same bits as
+    at the bottom of a low one, and a first call's host work that follows the
+    blocks, not the layers between them and below them (a fraction of a
+    millisecond; 98 ms with an item list walked layer by layer)."""
+    bsx, low, tall = 8, 24, 1 << 20
+    r = np.random.default_rng(7)
+    layers = np.array([4, 5, 6, 9, 17, 18])
+    values = r.uniform(0, 1, (len(layers), bsx ** 3)).astype(np.float32)
+    params = msbg.PdeParams(0.05, 10, False)
+    got, took = [], []
+    for height, up in ((low, 0), (tall, tall - low)):
+        g = msbg.SparseGrid(ctx, bsx, bsx, bsx * height, 0.25, 0.75, bsx)
+        ids = (layers + up).astype(np.uint64)
+        g.write_blocks(ids, values)
+        sw = msbg.Sweeper(g)
+        ctx.synchronize()
+        for turn in range(3):  # another active set each time: another plan
+            active = ids if turn == 0 else ids[turn:]
+            t0 = time.perf_counter()
+            sw.sweep(active, 0, params)
+            ctx.synchronize()
+            took.append(time.perf_counter() - t0)
+        got.append(g.read_blocks(ids))
+        if not up:  # a gap of a million layers between two blocks as well
+            g2 = msbg.SparseGrid(ctx, bsx, bsx, bsx * tall, 0.25, 0.75, bsx)
+            far = np.array([4, 5, 6, tall - low + 9, tall - low + 17, tall - low + 18], np.uint64)
+            g2.write_blocks(far, values)
+            for turn in range(3):
+                msbg.Sweeper(g2).sweep(far if turn == 0 else far[turn:], 0, params)
+            got.append(g2.read_blocks(far))
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+    assert min(took[3:]) < 0.03, took
