@@ -43,6 +43,7 @@ struct SplatArgs {
     double* partial;                         // [npb][3][2][W^3]
     int* status;                             // device status word (bit 4: a tile wait gave up)
     float r_p, inv_r2;
+    bool narrow;                             // the cell groups take compact_rows(r_p) rows, not all 2M+1
 };
 
 template <int BSX> struct P2GLg { static constexpr int v = BSX == 8 ? 3 : BSX == 16 ? 4 : 5; };
@@ -156,15 +157,17 @@ __global__ void cell_csr_kernel(const uint64_t* skeys, const uint64_t* pb_starts
 // dv - M along U and V, and bit 56 + s (s in [0, 2M]) when the face
 // footprint (offset 1.0) along F holds cell offset s - 1 - M.
 // MT > 0 fixes M = MT at compile time (the footprint loops unrolled).
-template <int MT>
+// EDGE: *edge += the particles with a row at either end of the 2M+1.
+template <int MT, bool EDGE>
 __global__ void p2g_gather_kernel(const float* pos, const float* vel, const float* mass, const uint32_t* perm, size_t n,
                                   int lg, int M_, float r_p, float r_scan_bsx, int64_t nx, int64_t ny, int64_t nz,
                                   float* px, float* py, float* pz, float* pm, float* v0, float* v1, float* v2,
-                                  uint32_t* fmask, uint64_t* lane_mask, int* bad) {
+                                  uint32_t* fmask, uint64_t* lane_mask, int* bad, unsigned int* edge) {
     const int M = MT > 0 ? MT : M_;
     const float inv_bsx = 1.0f / (float)(1 << lg);
     const int32_t B = 1 << lg;
     const int WIN = 2 * M + 1;
+    uint32_t n_edge = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t s = perm ? perm[i] : i;
         const float x = pos[3 * s], y = pos[3 * s + 1], z = pos[3 * s + 2];
@@ -213,6 +216,7 @@ __global__ void p2g_gather_kernel(const float* pos, const float* vel, const floa
                 const int lo = max(a1[ax][face] - cell[ax] + face, 0), hi = min(a2[ax][face] - cell[ax] + face, WIN - 1);
                 run[ax][face] = lo > hi ? 0u : ((2u << hi) - 1u) & ~((1u << lo) - 1u);
             }
+        if (EDGE) n_edge += ((run[0][0] | run[1][0] | run[2][0]) & (1u | (1u << (WIN - 1)))) != 0;
 #pragma unroll
         for (int dir = 0; dir < 3; ++dir) {
             const int F = dir, U = dir == 0 ? 1 : 0, V = dir == 2 ? 1 : 2;
@@ -246,6 +250,10 @@ __global__ void p2g_gather_kernel(const float* pos, const float* vel, const floa
         };
         const uint32_t xr = ((2u << hi[0]) - 1u) & ~((1u << lo[0]) - 1u);
         fmask[i] = xr * rep(lo[1], hi[1], 3) * rep(lo[2], hi[2], 9);
+    }
+    if (EDGE) {
+        n_edge = __reduce_add_sync(0xffffffffu, n_edge);
+        if ((threadIdx.x & 31) == 0 && n_edge) atomicAdd(edge, n_edge);
     }
 }
 
@@ -307,7 +315,7 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
 // Inside a tile, a group of RW^2 lanes takes a cell: the RW x RW rows of the
 // cell's face window across the two axes other than the face axis, RW being
 // the rows that a footprint of this radius covers unless a coordinate lies
-// exactly on a cell centre (compact_rows), so with RW = 3 a warp works on
+// exactly on a cell face (compact_rows), so with RW = 3 a warp works on
 // three cells at once (4.2 M particles in 16^3 blocks, r_p = 1.5, B200: 1.86 ms
 // with 25 rows of which 9 carry weight, 0.91 ms with 3 x 9; 5.6 M in 8^3
 // blocks 8.64 -> 1.71 ms with the smaller CTAs).  Each lane keeps the 2M+1 faces along
@@ -316,8 +324,9 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
 // the particle's clipped footprint (p2g.rs:263-330, operation by operation;
 // the footprint arrives as the particle's lane and face bits), then the groups
 // add their register sums to the window in cell order.  Rows of a footprint
-// beyond the RW x RW ones (a particle exactly on a cell centre) are added by
-// the whole warp after the cells.
+// beyond the RW x RW ones (a particle on a cell face, r_p - 1/2 an integer)
+// are added by the whole warp after the cells, one particle at a time; where
+// many particles have such rows RW is the whole window instead (kEdgeShare).
 // A tile wait that runs past a second sets bit 4 of the status word and goes
 // on (the result is then wrong and the host reports the error).
 template <int M, int RW> struct CellLanes {
@@ -1168,10 +1177,20 @@ static void launch_splat_cells(msbg_ctx* ctx, const SplatArgs& a, size_t npb) {
 }
 
 // Rows along a lane axis that a footprint of radius r_p covers about its cell
-// unless a coordinate lies exactly on a cell centre: a particle at fraction f
-// of its cell reaches ceil(f - r_p - 1/2) .. floor(f + r_p - 1/2), for 0 < f < 1
-// within -floor(r_p) .. ceil(r_p - 1/2) - that is -h .. h with h = ceil(r_p - 1/2).
+// unless a coordinate lies on a cell face (is an integer): a particle at
+// fraction f of its cell reaches ceil(f - r_p - 1/2) .. floor(f + r_p - 1/2), for
+// 0 < f < 1 within -h .. h with h = ceil(r_p - 1/2).  At f = 0 it reaches
+// -(h + 1) when r_p - 1/2 is an integer (1.5, 2.5), and so, by the rounding of
+// p - r_p, may one beside a face or of a radius close to these.
 static int compact_rows(float r_p) { return 2 * (int)ceilf(r_p - 0.5f) + 1; }
+
+// One particle in this many with rows beyond the compact ones, and the groups
+// take the whole window: a program that seeds its particles on integer
+// coordinates has them all there.  P2G, B200, compact against whole window by
+// the share of such particles: 4.8 M particles, 16^3 blocks, r_p = 1.5, none 1.11 /
+// 1.83 ms, a quarter 1.72 / 1.82, all 2.96 / 1.83; r_p = 2.5, none 3.5 / 5.5, a quarter
+// 6.3 / 5.5, all 13.0 / 5.5; 8^3 blocks, 1.5, a tenth 2.16 / 2.43, a quarter 2.62 / 2.43.
+constexpr size_t kEdgeShare = 5;
 
 template <int BSX, int M>
 static void launch_splat(msbg_ctx* ctx, const SplatArgs& a, size_t npb) {
@@ -1188,10 +1207,8 @@ static void launch_splat(msbg_ctx* ctx, const SplatArgs& a, size_t npb) {
         after_launch(ctx, "p2g_r2_kernel");
         return;
     }
-    // rows beyond these are added one particle at a time, so a narrower
-    // choice is always right and only slow when many particles need it
     if constexpr (M > 1) {
-        if (compact_rows(a.r_p) < 2 * M + 1) {
+        if (a.narrow) {
             launch_splat_cells<BSX, M, 2 * M - 1>(ctx, a, npb);
             return;
         }
@@ -1268,7 +1285,9 @@ void p2g_device(msbg_mac* mac, const float* d_pos, const float* d_vel, const flo
     uint64_t* pb_key = ScratchLayout::at<uint64_t>(base, o_pbk);
     uint64_t* pb_starts = ScratchLayout::at<uint64_t>(base, o_pbs);
     int* bad = ScratchLayout::at<int>(base, o_bad);
-    CUDA_CHECK(cudaMemsetAsync(bad, 0, 4, ctx->stream));
+    unsigned int* edge = reinterpret_cast<unsigned int*>(bad) + 1;  // particles with rows beyond the compact ones
+    const bool compact = M > 1 && compact_rows(r_p) < 2 * M + 1;
+    CUDA_CHECK(cudaMemsetAsync(bad, 0, 8, ctx->stream));
     if (d_sorted_keys) {
         skeys = d_sorted_keys;
         perm = const_cast<uint32_t*>(d_perm);
@@ -1279,25 +1298,27 @@ void p2g_device(msbg_mac* mac, const float* d_pos, const float* d_vel, const flo
     }
     float *px = soa, *py = soa + n, *pz = soa + 2 * n, *pm = soa + 3 * n, *v0 = soa + 4 * n, *v1 = soa + 5 * n, *v2 = soa + 6 * n;
     begin_launch(ctx);
-    if (M == 2)
-        p2g_gather_kernel<2><<<grid_for(n), 256, 0, ctx->stream>>>(d_pos, d_vel, d_mass, perm, n, lg, M, r_p,
-                                                                   (r_p + 1.0f) / (float)bsx, (int64_t)u->nx, (int64_t)u->ny,
-                                                                   (int64_t)u->nz, px, py, pz, pm, v0, v1, v2, fmask, fpk, bad);
-    else
-        p2g_gather_kernel<0><<<grid_for(n), 256, 0, ctx->stream>>>(d_pos, d_vel, d_mass, perm, n, lg, M, r_p,
-                                                                   (r_p + 1.0f) / (float)bsx, (int64_t)u->nx, (int64_t)u->ny,
-                                                                   (int64_t)u->nz, px, py, pz, pm, v0, v1, v2, fmask, fpk, bad);
+    auto gather = [&](auto kernel) {
+        kernel<<<grid_for(n), 256, 0, ctx->stream>>>(d_pos, d_vel, d_mass, perm, n, lg, M, r_p, (r_p + 1.0f) / (float)bsx,
+                                                     (int64_t)u->nx, (int64_t)u->ny, (int64_t)u->nz, px, py, pz, pm, v0, v1, v2,
+                                                     fmask, fpk, bad, edge);
+    };
+    if (M == 2 && compact) gather(p2g_gather_kernel<2, true>);
+    else if (M == 2) gather(p2g_gather_kernel<2, false>);
+    else if (compact) gather(p2g_gather_kernel<0, true>);
+    else gather(p2g_gather_kernel<0, false>);
     after_launch(ctx, "p2g_gather_kernel");
     const size_t npb = sorted_segments(ctx, skeys, n, (uint64_t)(3 * lg), pb_key, pb_starts, ScratchLayout::at<char>(base, o_tmp));
-    int hbad = 0, hstatus = 0;
+    int hbad[2] = {0, 0}, hstatus = 0;
     {
         SmallReads rd(ctx);
-        rd.add(&hbad, bad, 4);
+        rd.add(hbad, bad, 8);
         rd.add(&hstatus, ctx->status.p, 4);
         rd.wait();
     }
     raise_device_status(ctx, hstatus);
-    MSBG_REQUIRE(!hbad, "a particle lies outside the domain");
+    MSBG_REQUIRE(!hbad[0], "a particle lies outside the domain");
+    const bool narrow = compact && (size_t)(uint32_t)hbad[1] * kEdgeShare <= n;
 
     // ---- phase 2: active set ------------------------------------------------
     ScratchLayout L2 = L1;
@@ -1393,6 +1414,7 @@ void p2g_device(msbg_mac* mac, const float* d_pos, const float* d_vel, const flo
     s.partial = partial;
     s.r_p = r_p;
     s.inv_r2 = 1.0f / (r_p * r_p);
+    s.narrow = narrow;
     dispatch(ctx, bsx, M, &s, npb, nullptr, 0);
     CombineArgs c;
     c.partial = partial;
