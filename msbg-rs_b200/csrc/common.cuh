@@ -143,7 +143,19 @@ char* scratch(msbg_ctx* ctx, const ScratchLayout& L);
 // reads of data no kernel in flight writes then overlap the kernel before.
 // Data read after chain_wait must not come through `const __restrict__`
 // pointers: those reads may be moved ahead of it.
+// The trigger costs the chip about 1 ns a CTA, one after the other (B200: 202,256
+// CTAs of 64 threads 213 us with it, 111 us without), which counts where CTAs are
+// short and may be many, one to a small block.  Those call chain_trigger_short:
+// beyond kChainMaxCtas they leave it out and trigger as they end.  PCG on 12.9 M
+// cells in 4^3 blocks: 21.2 ms with the trigger in every grid, 17.5 ms with this
+// limit; 7-tap sweeps of 202,256 u16 blocks of 4^3 0.99 -> 0.73 ms.  Kernels whose
+// grids are capped or whose CTAs take microseconds trigger always: the test
+// alone costs 0.1 us a launch (5 19-tap sweeps of u16, 40 launches: 506 -> 510 us).
 __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+constexpr unsigned kChainMaxCtas = 4096;
+__device__ __forceinline__ void chain_trigger_short() {  // (one-dimensional grids)
+    if (gridDim.x <= kChainMaxCtas) chain_trigger();
+}
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // cluster > 1: thread-block clusters of that many CTAs along x.

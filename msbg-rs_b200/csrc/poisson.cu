@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(NT) pk_restrict_tile(TransferArgs T, const flo
     float* const f = reinterpret_cast<float*>(f2);
     __shared__ int32_t fs[27];
     const int64_t k = blockIdx.x;
-    chain_trigger();
+    chain_trigger_short();
     if (threadIdx.x < 27) {
         // fine block at offset (t % 3, t / 3 % 3, t / 9) - 1; the restriction table starts at offset -1
         const int t = threadIdx.x;
@@ -745,7 +745,7 @@ __global__ void __launch_bounds__(NT) pk_prolong_tile(TransferArgs T, const floa
     __shared__ float c[W * W * W];  // coarse cells -1 .. BC of fine block k's parent
     __shared__ int32_t cs[27];
     const int64_t k = blockIdx.x;
-    chain_trigger();
+    chain_trigger_short();
     if (threadIdx.x < 27) cs[threadIdx.x] = T.nb[k * 27 + threadIdx.x];
     __syncthreads();
     chain_wait();

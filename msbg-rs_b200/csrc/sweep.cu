@@ -623,7 +623,8 @@ sweep_phase_kernel(SweepArgs a, const int32_t* __restrict__ order) {
     typename E::T* payload = (typename E::T*)a.payload;
     const int tid = threadIdx.x, nthr = blockDim.x;
 
-    chain_trigger();
+    if (BSX >= 16) chain_trigger();
+    else chain_trigger_short();
     {
         const int t = blockIdx.x;  // one block per CTA
         const int pi = order[t];
