@@ -553,11 +553,11 @@ struct TransferArgs {
 };
 
 // Four lanes form a coarse cell: lane tz the four x-sums of its fine plane, which
-// lane 0 then adds plane by plane.  The levels this runs on are small (a few
+// lane 0 then adds plane by plane.  Most levels this runs on are small (a few
 // thousand cells), so it is bound by one thread's chain of address arithmetic
 // and loads: 16 of them instead of 64 (B200, solve of 3.18 M cells 2.56 -> 2.42
 // ms, 16 batched solves 4.88 -> 4.71).
-__global__ void pk_restrict(TransferArgs T, const float* r, float* __restrict__ bc) {
+__global__ void pk_restrict4(TransferArgs T, const float* r, float* __restrict__ bc) {
     chain_trigger();
     const int bsc = 1 << T.lgc, mc = bsc - 1, mf = (1 << T.lgf) - 1;
     const int tz = threadIdx.x & 3;
@@ -602,6 +602,57 @@ __global__ void pk_restrict(TransferArgs T, const float* r, float* __restrict__ 
     }
     if (!waited) chain_wait();
 }
+
+// The same with a thread per coarse cell, for the finest levels of 32^3 blocks:
+// there the chip is full and the lanes' repeated address arithmetic counts
+// (kRestrictLanesMax).
+__global__ void pk_restrict(TransferArgs T, const float* r, float* __restrict__ bc) {
+    chain_trigger();
+    chain_wait();
+    const int bsc = 1 << T.lgc, mc = bsc - 1, mf = (1 << T.lgf) - 1;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T.cells; i += (int64_t)gridDim.x * blockDim.x) {
+        if (T.diag && !(T.diag[i] > 0.0f)) {
+            bc[i] = 0.0f;
+            continue;
+        }
+        const int64_t k = i >> (3 * T.lgc);
+        const int v = (int)(i & ((1 << (3 * T.lgc)) - 1));
+        const int q[3] = {T.coords[3 * k] * bsc + (v & mc), T.coords[3 * k + 1] * bsc + ((v >> T.lgc) & mc),
+                          T.coords[3 * k + 2] * bsc + (v >> (2 * T.lgc))};
+        int fb0[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) fb0[a] = ((2 * T.coords[3 * k + a] * bsc) >> T.lgf) - 1;
+        const int32_t* nb = T.nb + k * 64;
+        const float w1[4] = {0.25f, 0.75f, 0.75f, 0.25f};
+        float s = 0.0f;
+#pragma unroll
+        for (int tz = 0; tz < 4; ++tz) {
+            const int gz = 2 * q[2] - 1 + tz, bz = (gz >> T.lgf) - fb0[2];
+#pragma unroll
+            for (int ty = 0; ty < 4; ++ty) {
+                const int gy = 2 * q[1] - 1 + ty, by = (gy >> T.lgf) - fb0[1];
+                float row = 0.0f;
+#pragma unroll
+                for (int tx = 0; tx < 4; ++tx) {
+                    const int gx = 2 * q[0] - 1 + tx, bx = (gx >> T.lgf) - fb0[0];
+                    const int32_t sl = nb[bx + 4 * by + 16 * bz];
+                    const float val = sl >= 0 ? r[((int64_t)sl << (3 * T.lgf)) + ((gx & mf) | ((gy & mf) << T.lgf) |
+                                                                                   ((gz & mf) << (2 * T.lgf)))]
+                                              : 0.0f;
+                    row += w1[tx] * val;
+                }
+                s += (w1[ty] * w1[tz]) * row;
+            }
+        }
+        bc[i] = s * 0.125f;
+    }
+}
+
+// Coarse cells up to which pk_restrict4 is taken.  B200, PCG on 32^3 blocks with it
+// against pk_restrict everywhere, by the coarse cells under the finest level:
+// 32,768 0.95 against 1.02 ms; 110,592 1.58 either way; 262,144 2.62 against 2.54;
+// 2,097,152 14.3 against 13.6.
+constexpr int64_t kRestrictLanesMax = 200000;
 
 // x_f += P x_c at the active fine cells.  As in each_cell, the first cell's
 // coarse cells are looked up (four dependent table reads) before the wait.
@@ -1266,7 +1317,10 @@ static void vcycle(msbg_poisson* P, int l, float* x, const float* b, bool x_zero
         else launch_chained(P->ctx->stream, pk_restrict_tile<2, 64>, nb, 64, 0, 1, R, F.r.as<float>(), C.b.as<float>());
         after_launch(P->ctx, "pk_restrict_tile");
     } else {
-        launch_chained(P->ctx->stream, pk_restrict, grid_for(4 * C.cells()), 256, 0, 1, R, F.r.as<float>(), C.b.as<float>());
+        if (C.cells() <= kRestrictLanesMax)
+            launch_chained(P->ctx->stream, pk_restrict4, grid_for(4 * C.cells()), 256, 0, 1, R, F.r.as<float>(), C.b.as<float>());
+        else
+            launch_chained(P->ctx->stream, pk_restrict, grid_for(C.cells()), 256, 0, 1, R, F.r.as<float>(), C.b.as<float>());
         after_launch(P->ctx, "pk_restrict");
     }
     vcycle(P, l + 1, C.x.as<float>(), C.b.as<float>(), true);
