@@ -40,3 +40,23 @@ def solve_twice(msbg, ctx, oracle, act, nb, bsx, method, mode, nu=(2, 2), oracle
 def test_restriction_of_the_finest_level(msbg, ctx, oracle, nb, bsx, count, mode):
     """196,608, 200,704 and 819,200 coarse cells under the finest level."""
     solve_twice(msbg, ctx, oracle, some_blocks(nb, count, count), nb, bsx, [msbg.MG, msbg.PCG][mode], mode)
+
+
+@pytest.mark.parametrize("nb,count", [(13, 2048), (13, 2049), (21, 8192), (21, 8193)])
+def test_tiles_and_dot_products_of_large_sets(msbg, ctx, oracle, nb, count):
+    """16^3 blocks on both sides of the quad tile's split and of the limit of
+    the dot products formed inside the kernels."""
+    solve_twice(msbg, ctx, oracle, some_blocks(nb, count, count), nb, 16, msbg.PCG, 1)
+
+
+SETS = [(1, 16, 1), (5, 16, 60), (9, 8, 300), (13, 16, 2049)]
+
+
+# (plain cycles diverge on the last set, in the FP64 oracle as well: it is left to CG)
+@pytest.mark.parametrize("nu,nb,bsx,count", [(nu, *q) for nu in [(1, 1), (2, 2), (3, 3)] for q in SETS] +
+                         [((1, 3), *q) for q in SETS[:3]])
+def test_smoother_counts(msbg, ctx, oracle, nu, nb, bsx, count):
+    """CG with odd and even sweep counts; with different counts before and
+    after, the cycle's post-sweeps end in the other buffer (plain cycles)."""
+    mode = 1 if nu[0] == nu[1] else 0
+    solve_twice(msbg, ctx, oracle, some_blocks(nb, count, nb), nb, bsx, [msbg.MG, msbg.PCG][mode], mode, nu)
