@@ -141,8 +141,10 @@ char* scratch(msbg_ctx* ctx, const ScratchLayout& L);
 // before it has finished with all its writes visible (and that one, having
 // waited itself, after every earlier one).  Launch latency, CTA start-up and
 // reads of data no kernel in flight writes then overlap the kernel before.
-// Data read after chain_wait must not come through `const __restrict__`
-// pointers: those reads may be moved ahead of it.
+// Data that kernels in flight write must not be read through `__restrict__`
+// pointers, const or not: nothing else, the wait included, is then taken to
+// change it, and the reads may be moved ahead of chain_wait.  Pointers that are
+// only written through, and those to tables no kernel writes, may have it.
 // The trigger costs the chip about 1 ns a CTA, one after the other (B200: 202,256
 // CTAs of 64 threads 213 us with it, 111 us without), which counts where CTAs are
 // short and may be many, one to a small block.  Those call chain_trigger_short:

@@ -231,7 +231,7 @@ __global__ void pk_residual64(LevelArgs L, const double* x, const float* b,
 }
 
 // x += a * d (x FP64, d f32)
-__global__ void pk_add64(int64_t n, double a, const float* d, double* __restrict__ x) {
+__global__ void pk_add64(int64_t n, double a, const float* d, double* x) {
     chain_trigger();
     chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -672,7 +672,7 @@ constexpr int64_t kRestrictLanesMax = 200000;
 
 // x_f += P x_c at the active fine cells.  As in each_cell, the first cell's
 // coarse cells are looked up (four dependent table reads) before the wait.
-__global__ void pk_prolong(TransferArgs T, const float* xc, float* __restrict__ xf) {
+__global__ void pk_prolong(TransferArgs T, const float* xc, float* xf) {
     chain_trigger();
     const int bsf = 1 << T.lgf, mf = bsf - 1, mc = (1 << T.lgc) - 1;
     int64_t at[8];
@@ -807,7 +807,7 @@ __global__ void __launch_bounds__(NT) pk_restrict_tile(TransferArgs T, const flo
 }
 
 template <int LGF, int NT>
-__global__ void __launch_bounds__(NT) pk_prolong_tile(TransferArgs T, const float* xc, float* __restrict__ xf) {
+__global__ void __launch_bounds__(NT) pk_prolong_tile(TransferArgs T, const float* xc, float* xf) {
     constexpr int BF = 1 << LGF, BC = BF / 2, LGC = LGF - 1, W = BC + 2, NF = BF * BF * BF;
     __shared__ float c[W * W * W];  // coarse cells -1 .. BC of fine block k's parent
     __shared__ int32_t cs[27];
@@ -912,7 +912,7 @@ __global__ void pk_axpby(int64_t n, float a, const float* x, float b, float* __r
 
 // Stage 2 of p.Ap (the same tree as pk_dot_final), then alpha = r.z / p.Ap.
 __global__ void __launch_bounds__(DOT_THREADS) pk_dot_final_alpha(const double* partial, int np,
-                                                                   double* __restrict__ sc) {
+                                                                   double* sc) {
     chain_trigger();
     chain_wait();
     __shared__ double sm[DOT_THREADS];
@@ -931,7 +931,7 @@ __global__ void __launch_bounds__(DOT_THREADS) pk_dot_final_alpha(const double* 
 // skipped on breakdown.  DOT: r.r of the new residual and the loop's test.
 template <bool DOT>
 __global__ void __launch_bounds__(256) pk_cg_update(int64_t n, const double* sc, const float* p,
-                                                    const float* q, double* __restrict__ x, float* __restrict__ r,
+                                                    const float* q, double* x, float* r,
                                                     DotArgs dot) {
     chain_trigger();
     chain_wait();
@@ -943,8 +943,9 @@ __global__ void __launch_bounds__(256) pk_cg_update(int64_t n, const double* sc,
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         float ri = r[i];
         if (!bad) {
+            const float qi = q[i];
             x[i] = fma(a, (double)p[i], x[i]);
-            ri = fmaf(na, q[i], ri);
+            ri = fmaf(na, qi, ri);
             r[i] = ri;
         }
         if (DOT) s += (double)ri * (double)ri;
@@ -952,7 +953,7 @@ __global__ void __launch_bounds__(256) pk_cg_update(int64_t n, const double* sc,
     if (DOT) dot_finish<256>(s, dot);
 }
 
-__global__ void pk_cg_beta(double* __restrict__ sc, int flexible) {
+__global__ void pk_cg_beta(double* sc, int flexible) {
     chain_trigger();
     chain_wait();
     cg_beta(sc, flexible);
@@ -960,7 +961,7 @@ __global__ void pk_cg_beta(double* __restrict__ sc, int flexible) {
 
 // p = z + beta p (f32; beta from the device; the product rounded, then the sum)
 __global__ void pk_cg_direction(int64_t n, const double* sc, const float* z,
-                                float* __restrict__ p) {
+                                float* p) {
     chain_trigger();
     chain_wait();
     const float b = (float)sc[SC_BETA];
@@ -988,7 +989,7 @@ static LevelArgs level_args(const PLevelDev& L) {
     return LevelArgs{L.nbr.as<int32_t>(), L.lg, L.cells(), L.scale, L.diag.p ? L.diag.as<float>() : nullptr};
 }
 
-__global__ void pk_solve_test(cudaGraphConditionalHandle h, const double* sc, SolveCtl* __restrict__ c,
+__global__ void pk_solve_test(cudaGraphConditionalHandle h, const double* sc, SolveCtl* c,
                               double* __restrict__ hist, int check_bad) {
     chain_trigger();
     chain_wait();
@@ -1265,7 +1266,8 @@ static void launch_residual(msbg_poisson* P, int l, const float* x, const float*
         after_launch(P->ctx, "pk_block16_residual");
         return;
     }
-    launch_chained(P->ctx->stream, pk_residual, shape_grid(L.cfg_res, L.cells()), kShapes[L.cfg_res].threads, 0, 1, level_args(L), x, b, r);
+    launch_chained(P->ctx->stream, pk_residual, shape_grid(L.cfg_res, L.cells()), kShapes[L.cfg_res].threads, 0, 1, level_args(L),
+                   x, b, r);
     after_launch(P->ctx, "pk_residual");
 }
 
@@ -1284,7 +1286,8 @@ static void jacobi(msbg_poisson* P, int l, float* x, const float* b, int sweeps,
             launch_block16<3>(P->ctx, L, L.slab, b, b, x, omega);
             after_launch(P->ctx, "pk_block16_jacobi0");
         } else {
-            launch_chained(P->ctx->stream, pk_jacobi_zero2, shape_grid(L.cfg_jac, L.cells()), kShapes[L.cfg_jac].threads, 0, 1, level_args(L), b, x, omega);
+            launch_chained(P->ctx->stream, pk_jacobi_zero2, shape_grid(L.cfg_jac, L.cells()), kShapes[L.cfg_jac].threads, 0, 1,
+                           level_args(L), b, x, omega);
             after_launch(P->ctx, "pk_jacobi_zero2");
         }
         s = 2;
@@ -1303,7 +1306,8 @@ static void jacobi(msbg_poisson* P, int l, float* x, const float* b, int sweeps,
             after_launch(P->ctx, "pk_block16_jacobi");
             continue;
         }
-        launch_chained(P->ctx->stream, pk_jacobi, shape_grid(L.cfg_jac, L.cells()), kShapes[L.cfg_jac].threads, 0, 1, level_args(L), (s == 0 && x_zero) ? nullptr : src, b, dst, omega);
+        launch_chained(P->ctx->stream, pk_jacobi, shape_grid(L.cfg_jac, L.cells()), kShapes[L.cfg_jac].threads, 0, 1,
+                       level_args(L), (s == 0 && x_zero) ? nullptr : src, b, dst, omega);
         after_launch(P->ctx, "pk_jacobi");
     }
     if (sweeps % 2 == 1) CUDA_CHECK(cudaMemcpyAsync(x, t, L.cells() * 4, cudaMemcpyDeviceToDevice, P->ctx->stream));
@@ -2141,7 +2145,7 @@ __device__ __forceinline__ void seg_scalars(double* S, int op, double tol2) {
 // problem), then the scalars that follow from it.  Launches bound these
 // kernels: with the scalars here and both updates in bk_update, three fewer per
 // iteration, the solve of 16 problems takes 5.24 instead of 5.30 ms (B200).
-__global__ void bk_seg_sum(int np, const int64_t* __restrict__ pb, const double* part, double* __restrict__ scal,
+__global__ void bk_seg_sum(int np, const int64_t* __restrict__ pb, const double* part, double* scal,
                            int slot, int op, double tol2) {
     chain_trigger();
     chain_wait();
@@ -2162,7 +2166,7 @@ __global__ void bk_seg_sum(int np, const int64_t* __restrict__ pb, const double*
 
 // p = z + beta_p p
 __global__ void bk_xpay(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* scal,
-                        const float* z, float* __restrict__ p) {
+                        const float* z, float* p) {
     chain_trigger();
     chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -2171,13 +2175,14 @@ __global__ void bk_xpay(int64_t n, int lg3, const int32_t* __restrict__ blk_prob
 
 // x64 += alpha_p p, r -= alpha_p q
 __global__ void bk_update(int64_t n, int lg3, const int32_t* __restrict__ blk_prob, const double* scal,
-                          const float* p, const float* q, double* __restrict__ x, float* __restrict__ r) {
+                          const float* p, const float* q, double* x, float* r) {
     chain_trigger();
     chain_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double alpha = scal[(int64_t)blk_prob[i >> lg3] * S_WIDTH + S_ALPHA];
+        const float qi = q[i], ri = r[i];
         x[i] += alpha * (double)p[i];
-        r[i] += (float)(-1.0f * alpha) * q[i];
+        r[i] = ri + (float)(-1.0f * alpha) * qi;
     }
 }
 
@@ -2287,9 +2292,11 @@ static void autotune(msbg_poisson* P) {
             for (int c = 0; c < kNumShapes; ++c) {
                 auto run = [&]() {
                     if (kind == 0)
-                        launch_chained(ctx->stream, pk_jacobi, shape_grid(c, cells), kShapes[c].threads, 0, 1, level_args(L), L.x.as<float>(), L.b.as<float>(), L.t.as<float>(), P->omega);
+                        launch_chained(ctx->stream, pk_jacobi, shape_grid(c, cells), kShapes[c].threads, 0, 1, level_args(L),
+                                       L.x.as<float>(), L.b.as<float>(), L.t.as<float>(), P->omega);
                     else
-                        launch_chained(ctx->stream, pk_residual, shape_grid(c, cells), kShapes[c].threads, 0, 1, level_args(L), L.x.as<float>(), L.b.as<float>(), L.r.as<float>());
+                        launch_chained(ctx->stream, pk_residual, shape_grid(c, cells), kShapes[c].threads, 0, 1, level_args(L),
+                                       L.x.as<float>(), L.b.as<float>(), L.r.as<float>());
                 };
                 run();
                 CUDA_CHECK(cudaEventRecord(e0, ctx->stream));
