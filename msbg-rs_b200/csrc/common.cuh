@@ -33,6 +33,7 @@ void set_last_error(const std::string& msg);
     do {                                                                                  \
         cudaError_t e_ = (expr);                                                          \
         if (e_ != cudaSuccess) {                                                          \
+            (void)cudaGetLastError(); /* reported here, not by the next launch's check */ \
             int code_ = (e_ == cudaErrorMemoryAllocation) ? MSBG_ERR_OOM : MSBG_ERR_CUDA; \
             MSBG_THROW(code_, std::string(#expr) + ": " + cudaGetErrorString(e_));        \
         }                                                                                 \
