@@ -1224,6 +1224,17 @@ template <int BSX, int ST, bool PAIR = true> struct CompactThreads {
 // blocks: 0.87 against 0.99 ms).
 constexpr int kPairMinPhaseBlocks = 1184;
 
+// When the next phase may start its CTAs (19 taps, 16^3 blocks, four CTAs an SM).
+// Early ones take places on whichever SMs have them: with SMs to spare they pile up
+// there and leave a part of the next phase's blocks waiting for each other, and with
+// two or three blocks a CTA the CTAs of three bunch.  So a CTA triggers as it
+// begins its last block, and after it when the phase's blocks fill at most
+// three of the four places.  B200, 10 sweeps, at once against as it stands: 2,800
+// blocks 0.86 / 0.72 ms (unchained 0.75), 4,000 0.87 / 0.87 (0.96), 7,200 1.70 / 1.60,
+// 12,000 2.49 / 2.37 (2.37), 24,000 4.15 / 4.19.  Pairs of columns for the 7 taps and 8^3
+// blocks trigger at once: 28,000 blocks of 8^3 0.50 / 0.54 ms.
+constexpr int kLateTriggerMax = 3 * 148;
+
 template <int BSX, int ST, bool CLAMP, bool PAIR>
 __global__ void __launch_bounds__(CompactThreads<BSX, ST, PAIR>::v, BSX == 16 ? 4 : 1)
 sweep_compact_kernel(SweepArgs a, const int32_t* __restrict__ order, int n) {
@@ -1257,7 +1268,8 @@ sweep_compact_kernel(SweepArgs a, const int32_t* __restrict__ order, int n) {
         }
     };
     int pi2 = 0;
-    chain_trigger();
+    constexpr bool LATE = BSX == 16 && ST == MSBG_MEAN_CURVATURE;  // see kLateTriggerMax
+    if (!LATE) chain_trigger();
     if (meta_thread) {
         int32_t nbv = 0, mv = 0;
         const int pi0 = order[t];
@@ -1279,6 +1291,7 @@ sweep_compact_kernel(SweepArgs a, const int32_t* __restrict__ order, int n) {
         const int sl = j % 3, sn = (j + 1) % 3, s2 = (j + 2) % 3;
         const int b = j & 1, bn = b ^ 1;
         const int tn = t + g, t2 = t + 2 * g, t3 = t + 3 * g;
+        if (LATE && tn >= n && n > kLateTriggerMax) chain_trigger();
         int32_t nb2 = 0, mv2 = 0;
         int pi3 = 0;
         if (meta_thread) {
@@ -1297,6 +1310,7 @@ sweep_compact_kernel(SweepArgs a, const int32_t* __restrict__ order, int n) {
         if (meta_thread && t2 < n) put_meta(s2, pi2, nb2, mv2);
         pi2 = pi3;
     }
+    if (LATE && n <= kLateTriggerMax) chain_trigger();
     cp_async_wait<0>();
 }
 

@@ -62,6 +62,8 @@ def test_phase_forms_density8(msbg, ctx, oracle, stencil, lanes):
 @pytest.mark.parametrize("dims,counts,stencil", [
     # the 19-tap stencil: clusters up to 296 blocks a phase, single columns above, pairs from 1,184 blocks
     ((320, 320, 320), [296, 297, 400, 60, 148, 1000, 1, 297], 1),
+    # (phases of at most 444 blocks let the next one in late)
+    ((320, 320, 320), [444, 445, 443, 446, 300, 592, 593, 444], 1),
     ((352, 352, 352), [1184, 1183, 1200, 1100, 1050, 1185, 1000, 1180], 1),
     # the 7-tap stencil: one launch up to 16,384 blocks, a kernel per phase above
     ((416, 416, 416), [2048] * 8, 0),
