@@ -97,11 +97,20 @@ __global__ void sf_fill_kernel(uint32_t* __restrict__ f, size_t n, uint32_t v) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) f[i] = v;
 }
 
-// Threads of a splat CTA, and the row pitch of its window: a warp covers 8
-// voxels along x of 4 rows, which lie on 32 different banks when the pitch is
-// 8 or 24 modulo 32.
+// Threads of a splat CTA, and the row pitch of its window, by the particles of
+// a block.  A warp covers 8 voxels along x of 4 rows, which lie on 32 different
+// banks when the pitch is 8 or 24 modulo 32; but padding makes a window up to
+// 2.4 times as large, and of a few particles' time most goes into clearing and
+// committing it, which many small CTAs an SM do best.  The kernel's time on a
+// shell in 256^3 (B200), 512 threads and the padded window against this choice,
+// 8^3 blocks, r_scan 0.75: 10 particles a block 30.5 / 17.4 us, 46 48.9 / 35.7; r_scan 5,
+// 46 182 / 168, 178 468 / 453; 16^3 blocks, 0.75: 14 16.4 / 14.6, 202 46.3 / 43.5.
 constexpr int kSplatThreads = 512;
-static int splat_pitch(int W) { return ((W + 7) / 16) * 16 + 8; }
+static int splat_threads(size_t per_block, int bsx) {
+    if (bsx >= 16) return per_block < 32 ? 256 : kSplatThreads;
+    return per_block < 16 ? 128 : per_block < 64 ? 256 : kSplatThreads;
+}
+static int splat_pitch(size_t per_block, int W) { return per_block < 256 ? W : ((W + 7) / 16) * 16 + 8; }
 // Few particle blocks leave SMs idle: their particles are split over this
 // many CTAs at most (each commits its own window).
 constexpr int kSplatMaxParts = 32;
@@ -412,7 +421,7 @@ static std::vector<uint64_t> surface_splat(msbg_grid* g, const float* d_pos, siz
     a.hash = device_hash(g);
     a.sx = (int64_t)g->sx; a.sy = (int64_t)g->sy; a.sz = (int64_t)g->sz;
     a.nx = (int64_t)g->nx; a.ny = (int64_t)g->ny;
-    a.lg = lg; a.m = m; a.W = W; a.P = splat_pitch(W);
+    a.lg = lg; a.m = m; a.W = W; a.P = splat_pitch(n / npb, W);
     a.r_scan = r_scan;
     a.dmax = r_scan * r_scan;
     a.inv = 1.0f / a.dmax;
@@ -424,7 +433,7 @@ static std::vector<uint64_t> surface_splat(msbg_grid* g, const float* d_pos, siz
     // particles a CTA on average: fewer do not pay for another window
     const size_t parts = std::min<size_t>({div_up(148 * 8, npb), std::max<size_t>(n / (npb * 1024), 1), kSplatMaxParts});
     begin_launch(ctx);
-    sf_splat_kernel<<<dim3((unsigned)npb, (unsigned)parts), kSplatThreads, smem, ctx->stream>>>(a);
+    sf_splat_kernel<<<dim3((unsigned)npb, (unsigned)parts), splat_threads(n / npb, bsx), smem, ctx->stream>>>(a);
     after_launch(ctx, "sf_splat_kernel");
     if (!active.empty()) {
         begin_launch(ctx);
