@@ -1210,9 +1210,11 @@ static void build(msbg_poisson* P, uint64_t sx, uint64_t sy, uint64_t sz, int bs
     sync(ctx);
 }
 
-// z-planes of a quad-tile CTA: 4 while that leaves the chip less than full
-// (776 blocks: a PCG solve 3.60 ms with 16, 3.50 ms with 4), 16 where whole
-// blocks fill it and splitting only re-reads planes.
+// z-planes of a quad-tile CTA: 4 while that leaves the chip less than full,
+// 16 where whole blocks fill it and splitting only re-reads planes.  B200, a PCG
+// solve with 4 against 16 by the blocks: 400 1.47 / 1.79 ms, 776 2.17 / 2.38, 1,200 2.71 /
+// 2.81, 1,600 3.35 / 3.35, 2,048 4.43 / 4.25, 4,800 10.16 / 9.91 (and above 2,048 the
+// fused dot products would have more than kFusedDotMax partials with 4).
 constexpr int64_t kQuadSplitMax = 2048;
 static int quad_planes(int64_t n_blocks) { return n_blocks <= kQuadSplitMax ? 4 : 16; }
 

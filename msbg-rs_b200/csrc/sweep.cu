@@ -1218,10 +1218,12 @@ template <int BSX, int ST, bool PAIR = true> struct CompactThreads {
 };
 
 // The 19-tap stencil takes two columns per thread in colour phases of at
-// least this many blocks (B200, 16^3 blocks: 10 sweeps of 56,056 blocks 9.2
-// against 10.5 ms), one column otherwise: a phase of a few hundred blocks is
-// bound by the latency of one block, which twice the threads shorten (776
-// blocks: 0.87 against 0.99 ms).
+// least this many blocks, one column otherwise: a phase of few blocks is
+// bound by the latency of one block, which twice the threads shorten.  B200, 10
+// sweeps, pairs against one column by the blocks of a phase: 8^3 blocks 200 0.33 / 0.28
+// ms, 600 0.45 / 0.36, 1,184 0.48 / 0.42, 1,500 0.475 / 0.53; 16^3 blocks 296 0.68 / 0.68,
+// 600 1.00 / 1.06, 1,184 1.78 / 1.88, 7,007 9.2 / 10.5.  (8^3 blocks set the limit;
+// 16^3 blocks alone would cross near 300.)
 constexpr int kPairMinPhaseBlocks = 1184;
 
 // When the next phase may start its CTAs (19 taps, 16^3 blocks, four CTAs an SM).
@@ -1562,7 +1564,10 @@ __global__ void __launch_bounds__(BSX * BSX) sweep_cluster_kernel(SweepArgs a, c
 }
 
 // Colour phases of at most this many blocks run one block per cluster of 4
-// CTAs (16^3 blocks, one-cell halos).
+// CTAs (16^3 blocks, one-cell halos).  B200, 10 19-tap sweeps, clusters against one
+// CTA a block by the blocks of a phase: 100 0.41 / 0.66 ms, 150 0.57 / 0.76, 200 0.70 /
+// 0.81, 296 0.93 / 0.68, 400 1.10 / 0.72: they cross between 200 and 296, the
+// limit (two blocks an SM) stands above that.
 constexpr int kClusterMaxPhaseBlocks = 296;
 
 template <int BSX, int ST, bool CLAMP>
@@ -1653,10 +1658,13 @@ static void launch_wave_laplacian(msbg_ctx* ctx, const SweepArgs& a, const int2*
 }
 
 // The one-launch sweep runs the 7-tap stencil on active sets of at most
-// this many blocks (measured on B200, 10 sweeps: 872 blocks 0.21 against
-// 0.51 ms for a kernel per phase, 3,464 blocks 0.47 against 0.66 ms, 14,248
-// blocks 1.67 against 1.70 ms, 56,056 blocks 6.46 against 4.82 ms; the
-// 19-tap stencil gains nothing measurable at any size).
+// this many blocks.  The limit was taken against a kernel per phase launched
+// one after the other (B200, 10 sweeps: 872 blocks 0.21 against 0.51 ms, 14,248
+// 1.67 against 1.70, 56,056 6.46 against 4.82).  Against the phases chained as they are
+// now: 16^3 blocks, 2,000 0.31 / 0.42 ms, 4,000 0.54 / 0.44, 8,000 1.01 / 0.92, 14,248
+// 1.72 / 1.36, 20,000 2.39 / 1.85; 8^3 blocks, 4,000 0.22 / 0.27, 8,000 0.33 / 0.29,
+// 16,384 0.54 / 0.36: the two cross near 3,000 and 6,500 blocks, and the limit
+// stands above both.  (The 19-tap stencil gains nothing measurable at any size.)
 constexpr size_t kWaveMaxBlocks = 16384;
 
 // The (sweep, plan index) items of `iterations` sweeps in wavefront order:
