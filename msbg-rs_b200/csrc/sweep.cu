@@ -1859,20 +1859,19 @@ static SweepPlan* get_plan(msbg_grid* g, msbg_grid* coarse, const uint8_t* level
     // the value blocks in colour-major Morton order, each once (dummy or
     // absent ones are skipped, solver.rs:196-199)
     std::vector<std::pair<uint64_t, uint64_t>> buckets[8];
-    std::vector<char> seen(g->n_slots(), 0), xside(g->n_slots(), 0);
+    std::vector<uint64_t> xside((g->n_slots() + 63) / 64, 0);  // a bit per slot: a few active blocks of a large grid are cheap too
     for (size_t k = 0; k < n; ++k) {
         uint64_t bid = active[k];
         MSBG_REQUIRE(bid < g->n_blocks, "active block id out of range");
-        const int32_t slot = code_of(bid);
-        if (slot < 0 || seen[slot]) continue;
-        seen[slot] = 1;
+        if (code_of(bid) < 0) continue;
         int64_t bx, by, bz;
         block_coords(g, bid, &bx, &by, &bz);
         buckets[(bx & 1) | ((by & 1) << 1) | ((bz & 1) << 2)].push_back({morton3(bx, by, bz), bid});
     }
     size_t total = 0;
     for (auto& bk : buckets) {
-        std::stable_sort(bk.begin(), bk.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+        std::sort(bk.begin(), bk.end());
+        bk.erase(std::unique(bk.begin(), bk.end()), bk.end());
         total += bk.size();
     }
     auto plan = new SweepPlan;
@@ -1955,7 +1954,7 @@ static SweepPlan* get_plan(msbg_grid* g, msbg_grid* coarse, const uint8_t* level
                     }
                 }
                 np[k] = code;
-                if (k % 3 != 1 && code >= 0) xside[code] = 1;
+                if (k % 3 != 1 && code >= 0) xside[(size_t)code >> 6] |= 1ull << (code & 63);
             }
             order[pi] = pi;
             ++pi;
@@ -1966,7 +1965,7 @@ static SweepPlan* get_plan(msbg_grid* g, msbg_grid* coarse, const uint8_t* level
     // slots read through x-planes: x-side neighbours (faces and edges) that are value blocks
     std::vector<int32_t> xs;
     for (size_t k = 0; k < xside.size(); ++k)
-        if (xside[k]) xs.push_back((int32_t)k);
+        for (uint64_t w = xside[k]; w; w &= w - 1) xs.push_back((int32_t)(64 * k + __builtin_ctzll(w)));
     plan->n_xslots = xs.size();
     if (!xs.empty()) {
         plan->xslots.reserve(xs.size() * 4);
