@@ -923,8 +923,14 @@ static void launch_wgrad(msbg_ctx* ctx, const ConvLevel& L, const uint16_t* x, c
             return false;
         }
     };
-    if (L.lg == 3 && from_halos(std::integral_constant<int, 3>())) return;
-    if (L.lg == 2 && from_halos(std::integral_constant<int, 2>())) return;
+    // A few blocks leave its few CTAs a block's latency each, and the many small
+    // CTAs of the gather kernel finish earlier (a call with its host round trip, B200,
+    // gather against halos: 4^3, 64 -> 64 channels, 8 blocks 30.9 / 33.9 us, 20
+    // 38.2 / 39.1, 40 54.1 / 47.2; 16 and 32 input channels in halos' favour from one
+    // block on; 8^3, 32 -> 32, one block 27.0 / 28.1, three 30.1 / 28.3).
+    const bool few = L.lg == 3 ? L.n_blocks < 2 : CIN >= 64 && L.n_blocks < 20;
+    if (!few && L.lg == 3 && from_halos(std::integral_constant<int, 3>())) return;
+    if (!few && L.lg == 2 && from_halos(std::integral_constant<int, 2>())) return;
     // about 4 CTAs per SM in total, each over a contiguous range of whole 64-cell chunks
     const int64_t chunks = std::max<int64_t>(1, (cells + kWgCells - 1) / kWgCells);
     const int parts = (int)std::min<int64_t>(chunks, std::max<int64_t>(1, 592 / MT));

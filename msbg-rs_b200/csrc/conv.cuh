@@ -28,7 +28,8 @@
 // runs with M = (tap, Cin) pairs, N = Cout, K = cells, operands MN-major
 // (16-byte rows of 8 channels of one cell), partial sums per cell range
 // reduced in a fixed order: as conv3_wgrad_halo_kernel from staged halos on
-// 8^3 and 4^3 blocks, as conv3_wgrad_kernel with gathered operands elsewhere.
+// 8^3 and 4^3 blocks, as conv3_wgrad_kernel with gathered operands elsewhere
+// and for a few blocks.
 #pragma once
 
 #include "common.cuh"
