@@ -106,23 +106,29 @@ __global__ void __launch_bounds__(256) p2g_combine_kernel(CombineArgs a) {
     }
 }
 
-// CTAs that share a particle block in the two kernels below, so that a few
-// blocks of many particles still fill the chip (56 blocks of 32,768, B200:
+// CTAs that share a particle block in the cell tables and footprint masks, so that a
+// few blocks of many particles still fill the chip (56 blocks of 32,768, B200:
 // cell_csr 55 -> under 13 us, the footprint masks and candidates 55 -> 15 us;
 // both within 5 % at 512 blocks, where one CTA per block already filled it).
+// A CTA that has its block alone clears the block's table itself and goes on to
+// the candidates: two memsets and a launch less, 6 us of a call of 300.
 static unsigned block_parts(size_t n, size_t npb) {
     return (unsigned)std::max<size_t>(1, std::min<size_t>({div_up(148 * 8, npb), n / (npb * 1024), 64}));
 }
 
 // Cell CSR of a particle block (CTA column blockIdx.y takes a part of it):
 // begin/end index of every cell (by local Morton code) in the sorted particle
-// order; cells without particles keep the zeros the arrays were set to.
+// order; cells without particles stay zero (set before, if CTAs share the block).
 __global__ void cell_csr_kernel(const uint64_t* skeys, const uint64_t* pb_starts, int lg, int32_t* cell_begin,
                                 int32_t* cell_end) {
     const int k = blockIdx.x;
     const int n_cells = 1 << (3 * lg);
     int32_t* cb = cell_begin + (size_t)k * n_cells;
     int32_t* ce = cell_end + (size_t)k * n_cells;
+    if (gridDim.y == 1) {
+        for (int i = threadIdx.x; i < n_cells; i += blockDim.x) cb[i] = ce[i] = 0;
+        __syncthreads();
+    }
     // particle indices fit int32 (the CSR stores them as int32); a key's
     // neighbours come from the adjacent lanes (the warp's and the part's end
     // lanes load theirs), every lane of the CTA taking the same rounds
@@ -1117,20 +1123,38 @@ __global__ void pb_mask_kernel(const uint32_t* fmask, const uint64_t* pb_starts,
     if ((threadIdx.x & 31) == 0 && m) atomicOr(pbmask + k, m);
 }
 
-// The masks expanded to candidate block ids (n_blocks = "none").
+// Candidate d of a block's 27 (n_blocks = "none") from its mask.
+__device__ __forceinline__ uint64_t candidate_block(uint32_t mask, uint64_t key, int d, int64_t nx, int64_t ny, int64_t nz) {
+    const int64_t X = (int64_t)compact3(key) + d % 3 - 1, Y = (int64_t)compact3(key >> 1) + (d / 3) % 3 - 1,
+                  Z = (int64_t)compact3(key >> 2) + d / 9 - 1;
+    return ((mask >> d) & 1u) && X >= 0 && Y >= 0 && Z >= 0 && X < nx && Y < ny && Z < nz
+               ? (uint64_t)X + (uint64_t)Y * nx + (uint64_t)Z * nx * ny
+               : (uint64_t)(nx * ny * nz);
+}
+
+// The masks expanded to candidate block ids.
 __global__ void pb_candidates_kernel(const uint32_t* pbmask, const uint64_t* pb_key, size_t npb, int64_t nx, int64_t ny,
                                      int64_t nz, uint64_t* cand) {
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < npb * 27; t += (size_t)gridDim.x * blockDim.x) {
-        const size_t k = t / 27;
-        const int d = (int)(t % 27);
-        const uint64_t key = pb_key[k];
-        const int64_t X = (int64_t)compact3(key) + d % 3 - 1, Y = (int64_t)compact3(key >> 1) + (d / 3) % 3 - 1,
-                      Z = (int64_t)compact3(key >> 2) + d / 9 - 1;
-        const bool on = (pbmask[k] >> d) & 1u;
-        cand[t] = on && X >= 0 && Y >= 0 && Z >= 0 && X < nx && Y < ny && Z < nz
-                      ? (uint64_t)X + (uint64_t)Y * nx + (uint64_t)Z * nx * ny
-                      : (uint64_t)(nx * ny * nz);
-    }
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < npb * 27; t += (size_t)gridDim.x * blockDim.x)
+        cand[t] = candidate_block(pbmask[t / 27], pb_key[t / 27], (int)(t % 27), nx, ny, nz);
+}
+
+// Both at once, a CTA to a block.
+__global__ void pb_mask_candidates_kernel(const uint32_t* fmask, const uint64_t* pb_starts, const uint64_t* pb_key, int64_t nx,
+                                          int64_t ny, int64_t nz, uint64_t* cand) {
+    const size_t k = blockIdx.x;
+    const uint32_t* f = fmask + pb_starts[k];
+    const uint32_t cnt = (uint32_t)(pb_starts[k + 1] - pb_starts[k]);  // particles of one block
+    __shared__ uint32_t all;
+    if (threadIdx.x == 0) all = 0;
+    __syncthreads();
+    uint32_t m = 0;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x) m |= f[i];
+    m = __reduce_or_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicOr(&all, m);
+    __syncthreads();
+    if (threadIdx.x < 27) cand[k * 27 + threadIdx.x] = candidate_block(all, pb_key[k], (int)threadIdx.x, nx, ny, nz);
 }
 
 // For every active block, the particle-block rank of each of its 27
@@ -1345,14 +1369,22 @@ void p2g_device(msbg_mac* mac, const float* d_pos, const float* d_vel, const flo
     int32_t* cell_end = cell_begin + npb * NC;
     double* partial = ScratchLayout::at<double>(base, o_part);
 
-    CUDA_CHECK(cudaMemsetAsync(pbmask, 0, npb * 4, ctx->stream));
-    begin_launch(ctx);
-    pb_mask_kernel<<<dim3((unsigned)npb, block_parts(n, npb)), 256, 0, ctx->stream>>>(fmask, pb_starts, pbmask);
-    after_launch(ctx, "pb_mask_kernel");
-    begin_launch(ctx);
-    pb_candidates_kernel<<<grid_for(npb * 27), 256, 0, ctx->stream>>>(pbmask, pb_key, npb, (int64_t)u->nx, (int64_t)u->ny,
-                                                                      (int64_t)u->nz, cand);
-    after_launch(ctx, "pb_candidates_kernel");
+    const unsigned parts = block_parts(n, npb);
+    if (parts == 1) {
+        begin_launch(ctx);
+        pb_mask_candidates_kernel<<<(unsigned)npb, 256, 0, ctx->stream>>>(fmask, pb_starts, pb_key, (int64_t)u->nx, (int64_t)u->ny,
+                                                                          (int64_t)u->nz, cand);
+        after_launch(ctx, "pb_mask_candidates_kernel");
+    } else {
+        CUDA_CHECK(cudaMemsetAsync(pbmask, 0, npb * 4, ctx->stream));
+        begin_launch(ctx);
+        pb_mask_kernel<<<dim3((unsigned)npb, parts), 256, 0, ctx->stream>>>(fmask, pb_starts, pbmask);
+        after_launch(ctx, "pb_mask_kernel");
+        begin_launch(ctx);
+        pb_candidates_kernel<<<grid_for(npb * 27), 256, 0, ctx->stream>>>(pbmask, pb_key, npb, (int64_t)u->nx, (int64_t)u->ny,
+                                                                          (int64_t)u->nz, cand);
+        after_launch(ctx, "pb_candidates_kernel");
+    }
     const int cbits = ilog2i(u->n_blocks + 1) + 1;
     radix_sort_pairs(ctx, cand, nullptr, csort, cperm, npb * 27, cbits, ScratchLayout::at<char>(base, o_ctmp));
     size_t nuniq = sorted_segments(ctx, csort, npb * 27, 0, act, ast, ScratchLayout::at<char>(base, o_ctmp));
@@ -1388,9 +1420,9 @@ void p2g_device(msbg_mac* mac, const float* d_pos, const float* d_vel, const flo
     int32_t* d_slots = ScratchLayout::at<int32_t>(base, o_sl);
     CUDA_CHECK(cudaMemcpyAsync(d_slots, slots.data(), na * 4, cudaMemcpyHostToDevice, ctx->stream));
 
-    CUDA_CHECK(cudaMemsetAsync(cell_begin, 0, 2 * npb * NC * 4, ctx->stream));
+    if (parts > 1) CUDA_CHECK(cudaMemsetAsync(cell_begin, 0, 2 * npb * NC * 4, ctx->stream));
     begin_launch(ctx);
-    cell_csr_kernel<<<dim3((unsigned)npb, block_parts(n, npb)), 256, 0, ctx->stream>>>(skeys, pb_starts, lg, cell_begin, cell_end);
+    cell_csr_kernel<<<dim3((unsigned)npb, parts), 256, 0, ctx->stream>>>(skeys, pb_starts, lg, cell_begin, cell_end);
     after_launch(ctx, "cell_csr_kernel");
     begin_launch(ctx);
     active_nbr_kernel<<<grid_for(na * 27), 256, 0, ctx->stream>>>(act, na, pb_key, npb, (int64_t)u->nx, (int64_t)u->ny,
